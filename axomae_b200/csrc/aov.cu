@@ -24,13 +24,20 @@ namespace {
 using namespace nb;
 
 struct AovParams {
-  int32_t W, H, vinv, kind;
+  int32_t W, H, vinv;
   uint32_t seed;
   float near_plane, far_plane;
   float inv_P[16], inv_V[16];
 };
 
-__global__ void k_aov(DevScene sc, const AovParams p, float4 *out) {
+/* Resident blocks of 128 threads per SM: the depth image is a walk alone, the others add shading. */
+template <int KIND>
+constexpr int kAovBlocks = KIND == NOVA_B200_AOV_DEPTH ? 10 : KIND == NOVA_B200_AOV_NORMAL ? 8 : 6;
+
+/* One kernel per BVH width and image: with every walk and all three images in one kernel it took 86
+ * registers, 5 resident blocks for a walk that waits on its node loads. */
+template <int WIDTH, int KIND>
+__global__ void __launch_bounds__(128, kAovBlocks<KIND>) k_aov(DevScene sc, const AovParams p, float4 *out) {
   const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
   if (pix >= (uint32_t)p.W * (uint32_t)p.H) return;
   const int y = (int)(pix / (uint32_t)p.W), x = (int)(pix - (uint32_t)y * (uint32_t)p.W);
@@ -44,10 +51,10 @@ __global__ void k_aov(DevScene sc, const AovParams p, float4 *out) {
   V4 d = mul(iP, V4{nx, ny, -1.f, 0.f});
   d = normalize(mul(iV, V4{d.x, d.y, -1.f, 0.f}));
   const V3 ro{o.x, o.y, o.z}, rd{d.x, d.y, d.z};
-  const TraceResult h = trace_closest(sc, ro, rd);
+  const TraceResult h = trace_closest_w<WIDTH>(sc, ro, rd);
   const uint32_t row = p.vinv ? (uint32_t)(p.H - 1 - y) : (uint32_t)y;
   float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (p.kind == NOVA_B200_AOV_DEPTH) {
+  if constexpr (KIND == NOVA_B200_AOV_DEPTH) {
     const float nr = p.near_plane, fr = p.far_plane;
     if (h.prim < 0) {
       res = make_float4(fr, fr, fr, fr);
@@ -61,7 +68,7 @@ __global__ void k_aov(DevScene sc, const AovParams p, float4 *out) {
     const DevInstance &I = sc.instances[__ldg(sc.prim_inst + h.prim)];
     const HitRecord hr = make_record(sc, ro, rd, I, (uint32_t)h.prim - I.prim_offset, h.t, h.u, h.v);
     const DevMaterial &mat = sc.materials[I.material];
-    if (p.kind == NOVA_B200_AOV_NORMAL) {
+    if constexpr (KIND == NOVA_B200_AOV_NORMAL) {
       const V3 ns = shading_normal(sc, hr, mat);
       res = make_float4(ns.x, ns.y, ns.z, 1.f);
     } else {
@@ -71,6 +78,17 @@ __global__ void k_aov(DevScene sc, const AovParams p, float4 *out) {
     }
   }
   out[(size_t)row * p.W + x] = res;
+}
+
+template <int WIDTH>
+void launch_aov(nova_b200_ctx *c, int32_t kind, const AovParams &p, float4 *out) {
+  const unsigned grid = (unsigned)(((size_t)p.W * p.H + 127) / 128);
+  if (kind == NOVA_B200_AOV_DEPTH)
+    k_aov<WIDTH, NOVA_B200_AOV_DEPTH><<<grid, 128, 0, c->stream>>>(c->scene, p, out);
+  else if (kind == NOVA_B200_AOV_NORMAL)
+    k_aov<WIDTH, NOVA_B200_AOV_NORMAL><<<grid, 128, 0, c->stream>>>(c->scene, p, out);
+  else
+    k_aov<WIDTH, NOVA_B200_AOV_EMISSIVE><<<grid, 128, 0, c->stream>>>(c->scene, p, out);
 }
 
 }  // namespace
@@ -90,7 +108,7 @@ extern "C" nova_b200_status nova_b200_render_aov(nova_b200_ctx *c, const nova_b2
     return fail(c, NOVA_B200_INVALID_ARGUMENT, "far_plane must exceed near_plane%s");
   cudaSetDevice(c->device);
   AovParams p{};
-  p.W = f->width, p.H = f->height, p.vinv = f->vertical_invert, p.kind = kind, p.seed = f->seed;
+  p.W = f->width, p.H = f->height, p.vinv = f->vertical_invert, p.seed = f->seed;
   p.near_plane = near_plane, p.far_plane = far_plane;
   for (int k = 0; k < 16; k++) p.inv_P[k] = f->inv_P[k], p.inv_V[k] = f->inv_V[k];
   const size_t npx = (size_t)f->width * f->height;
@@ -100,7 +118,12 @@ extern "C" nova_b200_status nova_b200_render_aov(nova_b200_ctx *c, const nova_b2
     NB_CUDA(c, cudaMallocAsync(&tmp, npx * sizeof(float4), c->stream), "cudaMalloc(aov film)");
     out = tmp;
   }
-  k_aov<<<(unsigned)((npx + 127) / 128), 128, 0, c->stream>>>(c->scene, p, out);
+  if (c->scene.width == 8)
+    launch_aov<8>(c, kind, p, out);
+  else if (c->scene.width == 1)
+    launch_aov<1>(c, kind, p, out);
+  else
+    launch_aov<2>(c, kind, p, out);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && film_host)
     e = cudaMemcpyAsync(film_host, out, npx * sizeof(float4), cudaMemcpyDeviceToHost, c->stream);

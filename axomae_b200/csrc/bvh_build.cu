@@ -167,10 +167,10 @@ __device__ void write_child(float4 *nodes, int node, int slot, const float lo[3]
   const float lx = pad_lo(lo[0]), ly = pad_lo(lo[1]), lz = pad_lo(lo[2]);
   const float hx = pad_hi(hi[0]), hy = pad_hi(hi[1]), hz = pad_hi(hi[2]);
   if (slot == 0) {
-    n[0] = lx, n[1] = hx, n[2] = ly, n[3] = hy;
+    n[0] = lx, n[1] = ly, n[2] = hx, n[3] = hy;
     n[8] = lz, n[9] = hz;
   } else {
-    n[4] = lx, n[5] = hx, n[6] = ly, n[7] = hy;
+    n[4] = lx, n[5] = ly, n[6] = hx, n[7] = hy;
     n[10] = lz, n[11] = hz;
   }
 }

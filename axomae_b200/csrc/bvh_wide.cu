@@ -42,8 +42,8 @@ __device__ __forceinline__ void read_children(const float4 *nodes2, uint32_t nod
   for (int s = 0; s < 2; s++) {
     Child c;
     c.ref = r[12 + s];
-    c.lo[0] = f[4 * s + 0], c.hi[0] = f[4 * s + 1];
-    c.lo[1] = f[4 * s + 2], c.hi[1] = f[4 * s + 3];
+    c.lo[0] = f[4 * s + 0], c.hi[0] = f[4 * s + 2];
+    c.lo[1] = f[4 * s + 1], c.hi[1] = f[4 * s + 3];
     c.lo[2] = f[8 + 2 * s], c.hi[2] = f[9 + 2 * s];
     if (c.lo[0] <= c.hi[0] && c.lo[1] <= c.hi[1] && c.lo[2] <= c.hi[2]) out[n++] = c; /* skip empty boxes */
   }
@@ -190,7 +190,7 @@ __global__ void k_collapse(const float4 *nodes2, const float4 *tris2, const WTas
   }
   for (int s = 0; s < 8; s++)
     for (uint32_t k = 0; k < leaf_cnt[s]; k++) {
-      const size_t src = 3 * (size_t)(leaf_first_[s] + k), dst = 3 * (size_t)(tri_base + leaf_off[s] + k);
+      const size_t src = kTriStride * (size_t)(leaf_first_[s] + k), dst = kTriStride * (size_t)(tri_base + leaf_off[s] + k);
       tris_out[dst] = tris2[src];
       tris_out[dst + 1] = tris2[src + 1];
       tris_out[dst + 2] = tris2[src + 2];

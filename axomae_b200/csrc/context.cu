@@ -261,7 +261,7 @@ __global__ void k_prim_boxes(nb::DevScene sc, const uint32_t *valid, uint32_t n,
 
 /* Triangle records in leaf order: (v0, prim id), (v1 - v0, instance), (v2 - v0, 0), object space. */
 __global__ void k_write_tris(nb::DevScene sc, const uint32_t *valid, const uint32_t *order, uint32_t n, float4 *tris) {
-  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  size_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t prim = valid[order[k]];
   const uint32_t inst = sc.prim_inst[prim];
@@ -271,9 +271,9 @@ __global__ void k_write_tris(nb::DevScene sc, const uint32_t *valid, const uint3
   const uint32_t a = m.idx[3 * tri], b = m.idx[3 * tri + 1], cc = m.idx[3 * tri + 2];
   const nb::V3 v0 = nb::vertex_position(m, a), v1 = nb::vertex_position(m, b), v2 = nb::vertex_position(m, cc);
   const nb::V3 e1 = v1 - v0, e2 = v2 - v0;
-  tris[3 * k + 0] = make_float4(v0.x, v0.y, v0.z, __int_as_float((int)prim));
-  tris[3 * k + 1] = make_float4(e1.x, e1.y, e1.z, __int_as_float((int)inst));
-  tris[3 * k + 2] = make_float4(e2.x, e2.y, e2.z, 0.f);
+  tris[nb::kTriStride * k + 0] = make_float4(v0.x, v0.y, v0.z, __int_as_float((int)prim));
+  tris[nb::kTriStride * k + 1] = make_float4(e1.x, e1.y, e1.z, __int_as_float((int)inst));
+  tris[nb::kTriStride * k + 2] = make_float4(e2.x, e2.y, e2.z, I.identity ? 1.f : 0.f);
 }
 
 /* Where one mesh's SoA attributes sit in the staging region and its 64 B records in the arena
@@ -451,15 +451,15 @@ __global__ void k_mesh_boxes(nb::DevMesh m, const uint32_t *ids, uint32_t n, flo
 
 /* Bottom-level triangle records in leaf order: (v0, mesh-local triangle id), (v1 - v0, 0), (v2 - v0, 0). */
 __global__ void k_write_blas_tris(nb::DevMesh m, const uint32_t *ids, const uint32_t *order, uint32_t n, float4 *tris) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t t = ids[order[k]];
   const uint32_t a = m.idx[3 * (size_t)t], b = m.idx[3 * (size_t)t + 1], cc = m.idx[3 * (size_t)t + 2];
   const nb::V3 v0 = nb::vertex_position(m, a), v1 = nb::vertex_position(m, b), v2 = nb::vertex_position(m, cc);
   const nb::V3 e1 = v1 - v0, e2 = v2 - v0;
-  tris[3 * k + 0] = make_float4(v0.x, v0.y, v0.z, __int_as_float((int)t));
-  tris[3 * k + 1] = make_float4(e1.x, e1.y, e1.z, 0.f);
-  tris[3 * k + 2] = make_float4(e2.x, e2.y, e2.z, 0.f);
+  tris[nb::kTriStride * k + 0] = make_float4(v0.x, v0.y, v0.z, __int_as_float((int)t));
+  tris[nb::kTriStride * k + 1] = make_float4(e1.x, e1.y, e1.z, 0.f);
+  tris[nb::kTriStride * k + 2] = make_float4(e2.x, e2.y, e2.z, 0.f);
 }
 
 /* A bottom level built at node 0 moved to node_base, its triangles to tri_base. */
@@ -483,8 +483,8 @@ __global__ void k_instance_boxes(const nb::DevInstance *inst, uint32_t n, const 
   const float4 *rn = nodes + 4 * (size_t)blas_root[I.mesh];
   const float4 n0 = rn[0], n1 = rn[1], n2 = rn[2];
   /* union of the root's two child boxes (an empty child box is inverted and drops out) */
-  const nb::V3 bl{fminf(n0.x, n1.x), fminf(n0.z, n1.z), fminf(n2.x, n2.z)};
-  const nb::V3 bh{fmaxf(n0.y, n1.y), fmaxf(n0.w, n1.w), fmaxf(n2.y, n2.w)};
+  const nb::V3 bl{fminf(n0.x, n1.x), fminf(n0.y, n1.y), fminf(n2.x, n2.z)};
+  const nb::V3 bh{fmaxf(n0.z, n1.z), fmaxf(n0.w, n1.w), fmaxf(n2.y, n2.w)};
   nb::V3 wl{FLT_MAX, FLT_MAX, FLT_MAX}, wh{-FLT_MAX, -FLT_MAX, -FLT_MAX};
   for (int k = 0; k < 8; k++) {
     const nb::V3 p{(k & 1) ? bh.x : bl.x, (k & 2) ? bh.y : bl.y, (k & 4) ? bh.z : bl.z};
@@ -576,10 +576,10 @@ nova_b200_status build_two_level(nova_b200_ctx *c, const nb::BvhBuildParams &p, 
   size_t scratch = n_inst;
   for (uint32_t m = 0; m < n_meshes; m++) scratch = std::max<size_t>(scratch, count[m]);
   cudaError_t e = cudaMallocAsync(&c->d_nodes, sizeof(float4) * 4 * total_nodes, c->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync(&c->d_tris, sizeof(float4) * 3 * total_tris, c->stream);
+  if (e == cudaSuccess) e = cudaMallocAsync(&c->d_tris, sizeof(float4) * (nb::kTriStride * total_tris + nb::kTriPad), c->stream);
   if (e == cudaSuccess) e = cudaMallocAsync(&c->d_blas_root, sizeof(uint32_t) * n_meshes, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->d_nodes, 0, sizeof(float4) * 4 * total_nodes, c->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_tris, 0, sizeof(float4) * 3 * total_tris, c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_tris, 0, sizeof(float4) * (nb::kTriStride * total_tris + nb::kTriPad), c->stream);
   if (e == cudaSuccess) e = cudaMallocAsync(&lo, sizeof(float4) * scratch, c->stream);
   if (e == cudaSuccess) e = cudaMallocAsync(&hi, sizeof(float4) * scratch, c->stream);
   if (e == cudaSuccess) e = cudaMallocAsync(&order, sizeof(uint32_t) * scratch, c->stream);
@@ -618,7 +618,7 @@ nova_b200_status build_two_level(nova_b200_ctx *c, const nb::BvhBuildParams &p, 
     const uint32_t n = count[m];
     const nb::DevMesh &M = c->h_meshes[m];
     float4 *nodes = c->d_nodes + 4 * (size_t)node_off[m];
-    float4 *tris = c->d_tris + 3 * (size_t)tri_off[m];
+    float4 *tris = c->d_tris + nb::kTriStride * (size_t)tri_off[m];
     k_mesh_boxes<<<(n + 255) / 256, 256, 0, c->stream>>>(M, ids[m], n, lo, hi);
     e = nb::build_bvh(lo, hi, n, p, nodes, order, c->stream, &r);
     if (e == cudaSuccess) {
@@ -1022,7 +1022,7 @@ nova_b200_status nova_b200_build_bvh(nova_b200_ctx *c, const nova_b200_bvh_optio
   float4 *d_lo = nullptr, *d_hi = nullptr;
   const size_t max_nodes = std::max<size_t>(2 * (size_t)n, 2);
   NB_CUDA(c, cudaMallocAsync(&c->d_nodes, sizeof(float4) * 4 * max_nodes, c->stream), "cudaMalloc(nodes)");
-  NB_CUDA(c, cudaMallocAsync(&c->d_tris, sizeof(float4) * 3 * (size_t)n, c->stream), "cudaMalloc(tris)");
+  NB_CUDA(c, cudaMallocAsync(&c->d_tris, sizeof(float4) * (nb::kTriStride * (size_t)n + nb::kTriPad), c->stream), "cudaMalloc(tris)");
   NB_CUDA(c, cudaMemsetAsync(c->d_nodes, 0, sizeof(float4) * 4 * max_nodes, c->stream), "memset(nodes)");
   NB_CUDA(c, cudaMallocAsync(&d_order, sizeof(uint32_t) * n, c->stream), "cudaMalloc(order)");
   NB_CUDA(c, cudaMallocAsync(&d_lo, sizeof(float4) * n, c->stream), "cudaMalloc(lo)");
@@ -1046,7 +1046,7 @@ nova_b200_status nova_b200_build_bvh(nova_b200_ctx *c, const nova_b200_bvh_optio
     float4 *wnodes = nullptr, *wtris = nullptr;
     NB_CUDA(c, cudaMallocAsync(&wnodes, sizeof(float4) * 5 * ((size_t)r.n_nodes + 1), c->stream),
             "cudaMalloc(wide nodes)");
-    cudaError_t we = cudaMallocAsync(&wtris, sizeof(float4) * 3 * (size_t)n, c->stream);
+    cudaError_t we = cudaMallocAsync(&wtris, sizeof(float4) * (nb::kTriStride * (size_t)n + nb::kTriPad), c->stream);
     if (we != cudaSuccess) {
       cudaFreeAsync(wnodes, c->stream);
       return cuda_fail(c, we, "cudaMalloc(wide triangles)");
@@ -1222,7 +1222,7 @@ nova_b200_status nova_b200_scene_info(nova_b200_ctx *c, uint64_t *tris, uint64_t
   if (leaves) *leaves = c->n_leaves;
   if (bytes)
     *bytes = c->scene_bytes + (uint64_t)c->n_nodes * (c->bvh_width == 8 ? 80 : 64) +
-             (uint64_t)c->n_valid * 48 + c->queue_bytes + c->radiance_cap * 16;
+             (uint64_t)c->n_valid * (16 * nb::kTriStride) + c->queue_bytes + c->radiance_cap * 16;
   return NOVA_B200_SUCCESS;
 }
 

@@ -1,11 +1,12 @@
 /* Device-resident scene layout.
  *
  * HBM layout (all arrays are owned by the context, see context.cu):
- *   tris       3 float4 per triangle in BVH leaf order: (v0.xyz, prim id), (e1.xyz, instance id), (e2.xyz, 0)
+ *   tris       3 float4 per triangle in BVH leaf order: (v0.xyz, prim id), (e1.xyz, instance id), (e2.xyz, 1 for an
+ *              identity instance, else 0)
  *              with object-space v0 and edges e1 = v1 - v0, e2 = v2 - v0 (Triangle.h:154-156 computes the
  *              same edges), 48 B per triangle.
  *   nodes      binary BVH, 4 float4 per node (64 B): both children's boxes and references
- *                n0 = (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y)   n1 = (c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y)
+ *                n0 = (c0.lo.x, c0.lo.y, c0.hi.x, c0.hi.y)   n1 = (c1.lo.x, c1.lo.y, c1.hi.x, c1.hi.y)
  *                n2 = (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z)   n3 = (ref0, ref1, count0, count1)
  *              ref >= 0: inner node index; ref < 0: leaf whose triangles start at ~ref (count in n3.z/w).
  *   prim_inst  instance index of every global primitive (primitive order of the reference:
@@ -17,6 +18,9 @@
 #include "dmath.cuh"
 
 namespace nb {
+
+constexpr int kTriStride = 3; /* float4 per triangle record */
+constexpr int kTriPad = 1;    /* float4 after the last one: a walk reads four from every record */
 
 struct DevTexture {
   const uint32_t *u8;

@@ -294,13 +294,12 @@ __device__ __forceinline__ unsigned warp_append(bool flag, unsigned *counter) {
  * on rays that hit.  At least 10 resident blocks of 128 (48 registers): the walk is latency-bound,
  * and 40 warps per SM beat 32 (-4% on the batched scenes); 12 blocks spill the walk state. */
 /* Resident blocks of 128 threads per SM that k_trace is compiled for (the register bound is
- * 65536 / (128 * blocks)): binary layouts and the 8-wide one separately. */
-#ifndef NB_TRACE_MIN_BLOCKS
-#define NB_TRACE_MIN_BLOCKS 10
-#endif
-#ifndef NB_TRACE8_MIN_BLOCKS
-#define NB_TRACE8_MIN_BLOCKS 10
-#endif
+ * 65536 / (128 * blocks)).  Binary: 10 blocks (48 registers, next to no spills), 21.6 ms of traversal
+ * on an 8-frame batch against 22.3 at 9 and 23.4 at 8.  Two-level: the walk also holds the world ray
+ * and the instance, so 10 blocks spill 150 B a thread: 5.3 ms on 1000 instances at 720p, 9 blocks
+ * (56 registers) 3.7 ms, 8 blocks 3.8. */
+template <int WIDTH>
+constexpr int kTraceBlocks = WIDTH == 1 ? 9 : 10;
 
 /* NB_HIT_CLASSES=1: the hit list holds non-transmissive hits from its front and transmissive ones
  * from its back (k_shade reads both ranges), so shading warps mostly run one lobe family: the
@@ -369,8 +368,9 @@ __device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, fl
 }
 
 template <int WIDTH, class JS, bool ADJ = false, bool COUNT = false>
-__global__ void __launch_bounds__(128, WIDTH == 8 ? NB_TRACE8_MIN_BLOCKS : NB_TRACE_MIN_BLOCKS) k_trace(Queue q, WaveCounters *wcp, float4 *hits, uint2 *hit_slot, float4 *L,
-                                               const __grid_constant__ JS js, const uint32_t *order = nullptr) {
+__global__ void __launch_bounds__(128, kTraceBlocks<WIDTH>)
+    k_trace(Queue q, WaveCounters *wcp, float4 *hits, uint2 *hit_slot, float4 *L,
+            const __grid_constant__ JS js, const uint32_t *order = nullptr) {
   const uint32_t n = wcp->n_active + wave_new(*wcp);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if ((i & ~31u) >= n) return; /* whole warps leave together (the append below is a warp ballot) */
@@ -1010,12 +1010,14 @@ __global__ void k_resolve(const float4 *L, uint32_t NP, uint32_t count, float4 *
   reinterpret_cast<float4 *>(out)[(size_t)row * W + x] = make_float4(a.x / denom, a.y / denom, a.z / denom, a.w / denom);
 }
 
-__global__ void k_trace_api(DevScene sc, uint64_t n, const float *o, const float *d, int32_t *prim, float *t, float *u,
-                            float *v) {
+/* One kernel per BVH width: with the three walks in one kernel the registers were the largest walk's. */
+template <int WIDTH>
+__global__ void __launch_bounds__(128, kTraceBlocks<WIDTH>)
+    k_trace_api(DevScene sc, uint64_t n, const float *o, const float *d, int32_t *prim, float *t, float *u, float *v) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const TraceResult r =
-      trace_closest(sc, V3{o[3 * i], o[3 * i + 1], o[3 * i + 2]}, V3{d[3 * i], d[3 * i + 1], d[3 * i + 2]});
+      trace_closest_w<WIDTH>(sc, V3{o[3 * i], o[3 * i + 1], o[3 * i + 2]}, V3{d[3 * i], d[3 * i + 1], d[3 * i + 2]});
   prim[i] = r.prim;
   t[i] = r.t;
   u[i] = r.u;
@@ -1903,7 +1905,13 @@ nova_b200_status nb_trace(nova_b200_ctx *c, uint64_t n, const float *o, const fl
   if (n == 0) return NOVA_B200_SUCCESS;
   if (!o || !d || !prim || !t || !u || !v) return fail(c, NOVA_B200_INVALID_ARGUMENT, "null buffer%s");
   cudaSetDevice(c->device);
-  k_trace_api<<<(unsigned)((n + 127) / 128), 128, 0, c->stream>>>(c->scene, n, o, d, prim, t, u, v);
+  const unsigned grid = (unsigned)((n + 127) / 128);
+  if (c->scene.width == 8)
+    k_trace_api<8><<<grid, 128, 0, c->stream>>>(c->scene, n, o, d, prim, t, u, v);
+  else if (c->scene.width == 1)
+    k_trace_api<1><<<grid, 128, 0, c->stream>>>(c->scene, n, o, d, prim, t, u, v);
+  else
+    k_trace_api<2><<<grid, 128, 0, c->stream>>>(c->scene, n, o, d, prim, t, u, v);
   NB_CUDA(c, cudaGetLastError(), "k_trace_api");
   NB_CUDA(c, cudaStreamSynchronize(c->stream), "trace");
   return NOVA_B200_SUCCESS;

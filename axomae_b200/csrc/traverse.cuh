@@ -25,21 +25,6 @@ namespace nb {
 
 constexpr int kTraversalStack = 64;
 
-/* When both children of a binary node are hit, the deferred one's node record is prefetched into L1
- * (NB_TRACE_PREFETCH=1) so the pop later finds it near. */
-#ifndef NB_TRACE_PREFETCH
-#define NB_TRACE_PREFETCH 0
-#endif
-/* Leaves are tested one triangle per loop iteration (NB_LEAF_STEP=1): on the 32-job batch this took
- * the traversal from 193 to 179 ms per step against whole leaves per iteration. */
-#ifndef NB_LEAF_STEP
-#define NB_LEAF_STEP 1
-#endif
-NB_D void prefetch_node(const float4 *nodes, int32_t ref) {
-#if NB_TRACE_PREFETCH
-  if (ref >= 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(nodes + 4 * (size_t)ref));
-#endif
-}
 constexpr float kRayTNear = 0.000001f; /* Ray::tnear, ray/Ray.h:14 */
 constexpr float kFarScale = 1.000000477f; /* 1 + 2^-21: covers the rounding of the slab distances */
 
@@ -79,102 +64,138 @@ NB_D float safe_rcp(float d) {
   return fabsf(d) > 1e-30f ? __frcp_rn(d) : copysignf(big, d);
 }
 
-/* Closest hit of one world-space ray on the binary BVH. */
+/* Two single-precision operations in one instruction (add / mul .f32x2, sm_100): each half rounds like
+ * the scalar operation. */
+NB_D uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+NB_D void unpack2(uint64_t p, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+NB_D uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+NB_D uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+/* A ray as the slab tests read it: (-origin) and the reciprocal direction, in the pairs of the node
+ * layout. */
+struct SlabRay {
+  uint64_t nxy, nzz, ixy, izz;
+  NB_D void set(V3 o, V3 d) {
+    const float iz = safe_rcp(d.z);
+    nxy = pack2(-o.x, -o.y);
+    nzz = pack2(-o.z, -o.z);
+    ixy = pack2(safe_rcp(d.x), safe_rcp(d.y));
+    izz = pack2(iz, iz);
+  }
+};
+
+/* The 64 bytes at a node or at a triangle (whose record is the first 48; the triangle array ends with
+ * kTriPad so that the last one's read stays inside). */
+struct Rec {
+  float4 q0, q1, q2, q3;
+};
+NB_D Rec load_rec(const float4 *p) { return {__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3)}; }
+
+/* Entry and exit distance of one child box: slabs as (plane - origin) * rcp(dir), two roundings per
+ * distance, the far end widened by 2^-21. */
+NB_D void slab(const SlabRay &r, uint64_t lo_xy, uint64_t hi_xy, uint64_t z, float tmax, float &tn, float &tf) {
+  float ax, ay, bx, by, az, bz;
+  unpack2(mul2(add2(lo_xy, r.nxy), r.ixy), ax, ay);
+  unpack2(mul2(add2(hi_xy, r.nxy), r.ixy), bx, by);
+  unpack2(mul2(add2(z, r.nzz), r.izz), az, bz);
+  tn = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fmaxf(fminf(az, bz), 0.f));
+  tf = fminf(fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz)) * kFarScale, tmax);
+}
+
+/* Visits an inner node: the nearer hit child becomes `cur`, the other goes on the stack; false when
+ * neither is hit. */
+NB_D bool visit_inner(const Rec &n, const SlabRay &sr, float tmax, int32_t *stack, int &sp, int32_t &cur) {
+  float c0n, c0f, c1n, c1f;
+  slab(sr, pack2(n.q0.x, n.q0.y), pack2(n.q0.z, n.q0.w), pack2(n.q2.x, n.q2.y), tmax, c0n, c0f);
+  slab(sr, pack2(n.q1.x, n.q1.y), pack2(n.q1.z, n.q1.w), pack2(n.q2.z, n.q2.w), tmax, c1n, c1f);
+  const bool h0 = c0n <= c0f, h1 = c1n <= c1f;
+  const int32_t r0 = __float_as_int(n.q3.x), r1 = __float_as_int(n.q3.y);
+  if (h0 && h1) {
+    const bool swap = c1n < c0n;
+    if (sp < kTraversalStack) stack[sp++] = swap ? r0 : r1;
+    cur = swap ? r1 : r0;
+    return true;
+  }
+  cur = h0 ? r0 : r1;
+  return h0 || h1;
+}
+
+/* Tests the record's triangle at tmax or nearer. */
+NB_D bool visit_tri(const Rec &q, V3 o, V3 d, float tmax, float &t, float &u, float &v) {
+  return mt_hit(o, d, V3{q.q0.x, q.q0.y, q.q0.z}, V3{q.q1.x, q.q1.y, q.q1.z}, V3{q.q2.x, q.q2.y, q.q2.z}, kRayTNear, tmax,
+                t, u, v);
+}
+
+/* Closest hit of one world-space ray on the binary BVH.
+ *
+ * Bound by instruction issue at 17 of 32 active lanes and by the latency of dependent loads (issue
+ * slots 67 % used on full waves; L1 60 %, DRAM 12 %).  One iteration visits a node or one triangle of a
+ * leaf, and both kinds of lane load their record before the branch: a warp with lanes of each kind
+ * waits for one load instead of two.  The slab distances are packed pairs (12 instructions a node
+ * instead of 24), and a leaf's identity flag comes with its triangle instead of from the instance
+ * table.  8 frames, 162 M rays: 24.5 -> 21.6 ms; 1 M incoherent rays on 65 k triangles (one call):
+ * 303 -> 253 us.  Slower: waiting until 4 or 8 lanes are in leaves (24.2 / 24.8 ms), converging the
+ * warp every iteration (25.1), whole leaves before the next node (23.3), lanes taking new rays from a
+ * pool of 64 to 128 (28.3 at best); equal: one 32-byte load per half record (21.9). */
 NB_D TraceResult trace_closest2(const DevScene &sc, V3 o, V3 d, uint64_t *node_visits = nullptr,
                                uint64_t *tri_tests = nullptr) {
   TraceResult r{-1, 0.f, 0.f, 0.f, 0u};
   float tmax = FLT_MAX; /* native.cpp:57 starts from MAXFLOAT */
-  const float ix = safe_rcp(d.x), iy = safe_rcp(d.y), iz = safe_rcp(d.z);
+  SlabRay sr;
+  sr.set(o, d);
   int32_t stack[kTraversalStack];
   int sp = 0;
   int32_t cur = 0; /* the root is always an inner node (a one-leaf scene gets an empty sibling) */
-  int32_t cached_inst = -1;
+  int32_t cached_inst = -1; /* the instance lo_o, lo_d are transformed into (-1: the world ray) */
   V3 lo_o = o, lo_d = d;
-  uint64_t nv = 0, tt = 0;
-#if NB_LEAF_STEP
-  uint32_t lk = 0, le = 0; /* the current leaf's next and end triangle */
-#endif
+  uint32_t nv = 0, tt = 0;
   for (;;) {
-    if (cur >= 0) {
+    const bool inner = cur >= 0;
+    const Rec q = load_rec(inner ? sc.nodes + 4 * (size_t)(uint32_t)cur : sc.tris + kTriStride * (size_t)leaf_first(cur));
+    if (inner) {
       nv++;
-      const float4 n0 = __ldg(&sc.nodes[4 * cur + 0]);
-      const float4 n1 = __ldg(&sc.nodes[4 * cur + 1]);
-      const float4 n2 = __ldg(&sc.nodes[4 * cur + 2]);
-      const float4 n3 = __ldg(&sc.nodes[4 * cur + 3]);
-      /* slabs as (plane - origin) * rcp(dir): two roundings per distance, far end widened by 2^-21 */
-      float a0 = (n0.x - o.x) * ix, b0 = (n0.y - o.x) * ix;
-      float a1 = (n0.z - o.y) * iy, b1 = (n0.w - o.y) * iy;
-      float a2 = (n2.x - o.z) * iz, b2 = (n2.y - o.z) * iz;
-      float c0n = fmaxf(fmaxf(fminf(a0, b0), fminf(a1, b1)), fmaxf(fminf(a2, b2), 0.f));
-      float c0f = fminf(fminf(fminf(fmaxf(a0, b0), fmaxf(a1, b1)), fmaxf(a2, b2)) * kFarScale, tmax);
-      float d0 = (n1.x - o.x) * ix, e0 = (n1.y - o.x) * ix;
-      float d1 = (n1.z - o.y) * iy, e1 = (n1.w - o.y) * iy;
-      float d2 = (n2.z - o.z) * iz, e2 = (n2.w - o.z) * iz;
-      float c1n = fmaxf(fmaxf(fminf(d0, e0), fminf(d1, e1)), fmaxf(fminf(d2, e2), 0.f));
-      float c1f = fminf(fminf(fminf(fmaxf(d0, e0), fmaxf(d1, e1)), fmaxf(d2, e2)) * kFarScale, tmax);
-      const bool h0 = c0n <= c0f, h1 = c1n <= c1f;
-      const int32_t r0 = __float_as_int(n3.x), r1 = __float_as_int(n3.y);
-      if (h0 && h1) {
-        int32_t first = r0, second = r1;
-        if (c1n < c0n) {
-          first = r1;
-          second = r0;
-        }
-        prefetch_node(sc.nodes, second);
-        if (sp < kTraversalStack) stack[sp++] = second;
-        cur = first;
-        continue;
-      } else if (h0) {
-        cur = r0;
-        continue;
-      } else if (h1) {
-        cur = r1;
-        continue;
-      }
+      if (visit_inner(q, sr, tmax, stack, sp, cur)) continue;
     } else {
-#if NB_LEAF_STEP
-      /* one triangle per loop iteration: a lane in a leaf costs its warp one triangle test per
-       * iteration, not the whole leaf, while the other lanes visit nodes */
-      if (lk >= le) {
-        lk = leaf_first(cur);
-        le = lk + leaf_count(cur);
-      }
-      {
-        const uint32_t k = lk++;
-#else
-      const uint32_t first = leaf_first(cur), count = leaf_count(cur);
-      for (uint32_t k = first; k < first + count; k++) {
-#endif
-        const float4 t0 = __ldg(&sc.tris[3 * k + 0]);
-        const float4 t1 = __ldg(&sc.tris[3 * k + 1]);
-        const float4 t2 = __ldg(&sc.tris[3 * k + 2]);
-        const int32_t inst = __float_as_int(t1.w);
-        if (inst != cached_inst) {
-          cached_inst = inst;
-          const DevInstance &I = sc.instances[inst];
-          if (I.identity) {
-            lo_o = o;
-            lo_d = d;
-          } else {
-            lo_o = xform_point(I.inv, o);
-            lo_d = xform_dir(I.inv, d);
-          }
+      const int32_t inst = __float_as_int(q.q1.w);
+      if (q.q2.w != 0.f) { /* an identity instance: the world ray bit for bit */
+        if (cached_inst >= 0) {
+          cached_inst = -1;
+          lo_o = o;
+          lo_d = d;
         }
-        tt++;
-        float ht, hu, hv;
-        if (mt_hit(lo_o, lo_d, V3{t0.x, t0.y, t0.z}, V3{t1.x, t1.y, t1.z}, V3{t2.x, t2.y, t2.z}, kRayTNear, tmax, ht,
-                   hu, hv)) {
-          tmax = ht;
-          r.prim = __float_as_int(t0.w);
-          r.inst = (uint32_t)inst;
-          r.t = ht;
-          r.u = hu;
-          r.v = hv;
-        }
+      } else if (inst != cached_inst) {
+        cached_inst = inst;
+        const DevInstance &I = sc.instances[inst];
+        lo_o = xform_point(I.inv, o);
+        lo_d = xform_dir(I.inv, d);
       }
-#if NB_LEAF_STEP
-      if (lk < le) continue;
-#endif
+      tt++;
+      float ht, hu, hv;
+      if (visit_tri(q, lo_o, lo_d, tmax, ht, hu, hv)) {
+        tmax = ht;
+        r.prim = __float_as_int(q.q0.w);
+        r.inst = (uint32_t)inst;
+        r.t = ht;
+        r.u = hu;
+        r.v = hv;
+      }
+      /* the leaf's next triangle: first + 1, count - 1 in the reference's code */
+      if ((~cur & 15) != 0) {
+        cur -= 15;
+        continue;
+      }
     }
     if (sp == 0) break;
     cur = stack[--sp];
@@ -190,9 +211,9 @@ NB_D void test_triangles(const S &sc, uint32_t first, uint32_t count, V3 o, V3 d
                          V3 &lo_d, float &tmax, TraceResult &r) {
   /* count: the caller counts triangle tests (trace_closest8's tri_tests) */
   for (uint32_t k = first; k < first + count; k++) {
-    const float4 t0 = __ldg(&sc.tris[3 * k + 0]);
-    const float4 t1 = __ldg(&sc.tris[3 * k + 1]);
-    const float4 t2 = __ldg(&sc.tris[3 * k + 2]);
+    const float4 t0 = __ldg(&sc.tris[kTriStride * k + 0]);
+    const float4 t1 = __ldg(&sc.tris[kTriStride * k + 1]);
+    const float4 t2 = __ldg(&sc.tris[kTriStride * k + 2]);
     const int32_t inst = __float_as_int(t1.w);
     if (inst != cached_inst) {
       cached_inst = inst;
@@ -261,13 +282,13 @@ struct Walk2 {
       const float4 n1 = __ldg(&sc.nodes[4 * cur + 1]);
       const float4 n2 = __ldg(&sc.nodes[4 * cur + 2]);
       const float4 n3 = __ldg(&sc.nodes[4 * cur + 3]);
-      const float a0 = (n0.x - o.x) * ix, b0 = (n0.y - o.x) * ix;
-      const float a1 = (n0.z - o.y) * iy, b1 = (n0.w - o.y) * iy;
+      const float a0 = (n0.x - o.x) * ix, b0 = (n0.z - o.x) * ix;
+      const float a1 = (n0.y - o.y) * iy, b1 = (n0.w - o.y) * iy;
       const float a2 = (n2.x - o.z) * iz, b2 = (n2.y - o.z) * iz;
       const float c0n = fmaxf(fmaxf(fminf(a0, b0), fminf(a1, b1)), fmaxf(fminf(a2, b2), 0.f));
       const float c0f = fminf(fminf(fminf(fmaxf(a0, b0), fmaxf(a1, b1)), fmaxf(a2, b2)) * kFarScale, tmax);
-      const float d0 = (n1.x - o.x) * ix, e0 = (n1.y - o.x) * ix;
-      const float d1 = (n1.z - o.y) * iy, e1 = (n1.w - o.y) * iy;
+      const float d0 = (n1.x - o.x) * ix, e0 = (n1.z - o.x) * ix;
+      const float d1 = (n1.y - o.y) * iy, e1 = (n1.w - o.y) * iy;
       const float d2 = (n2.z - o.z) * iz, e2 = (n2.w - o.z) * iz;
       const float c1n = fmaxf(fmaxf(fminf(d0, e0), fminf(d1, e1)), fmaxf(fminf(d2, e2), 0.f));
       const float c1f = fminf(fminf(fminf(fmaxf(d0, e0), fmaxf(d1, e1)), fmaxf(d2, e2)) * kFarScale, tmax);
@@ -403,57 +424,22 @@ NB_D TraceResult trace_closest_tl(const DevScene &sc, V3 o, V3 d, uint64_t *node
   TraceResult r{-1, 0.f, 0.f, 0.f, 0u};
   float tmax = FLT_MAX;
   V3 ro = o, rd = d;
-  float ix = safe_rcp(d.x), iy = safe_rcp(d.y), iz = safe_rcp(d.z);
+  SlabRay sr;
+  sr.set(o, d);
   int32_t stack[kTraversalStack];
   int sp = 0;
   int32_t cur = 0;
   uint32_t prim_base = 0, inst_in = 0;
-#if NB_LEAF_STEP
-  uint32_t lk = 0, le = 0; /* the current bottom-level leaf's next and end triangle */
-#endif
   bool inside = false;
   uint32_t nv = 0, tt = 0;
   for (;;) {
-    if (cur >= 0) {
-      nv++;
-      const float4 n0 = __ldg(&sc.nodes[4 * cur + 0]);
-      const float4 n1 = __ldg(&sc.nodes[4 * cur + 1]);
-      const float4 n2 = __ldg(&sc.nodes[4 * cur + 2]);
-      const float4 n3 = __ldg(&sc.nodes[4 * cur + 3]);
-      float a0 = (n0.x - ro.x) * ix, b0 = (n0.y - ro.x) * ix;
-      float a1 = (n0.z - ro.y) * iy, b1 = (n0.w - ro.y) * iy;
-      float a2 = (n2.x - ro.z) * iz, b2 = (n2.y - ro.z) * iz;
-      float c0n = fmaxf(fmaxf(fminf(a0, b0), fminf(a1, b1)), fmaxf(fminf(a2, b2), 0.f));
-      float c0f = fminf(fminf(fminf(fmaxf(a0, b0), fmaxf(a1, b1)), fmaxf(a2, b2)) * kFarScale, tmax);
-      float d0 = (n1.x - ro.x) * ix, e0 = (n1.y - ro.x) * ix;
-      float d1 = (n1.z - ro.y) * iy, e1 = (n1.w - ro.y) * iy;
-      float d2 = (n2.z - ro.z) * iz, e2 = (n2.w - ro.z) * iz;
-      float c1n = fmaxf(fmaxf(fminf(d0, e0), fminf(d1, e1)), fmaxf(fminf(d2, e2), 0.f));
-      float c1f = fminf(fminf(fminf(fmaxf(d0, e0), fmaxf(d1, e1)), fmaxf(d2, e2)) * kFarScale, tmax);
-      const bool h0 = c0n <= c0f, h1 = c1n <= c1f;
-      const int32_t r0 = __float_as_int(n3.x), r1 = __float_as_int(n3.y);
-      if (h0 && h1) {
-        int32_t first = r0, second = r1;
-        if (c1n < c0n) {
-          first = r1;
-          second = r0;
-        }
-        if (sp < kTraversalStack) stack[sp++] = second;
-        cur = first;
-        continue;
-      } else if (h0) {
-        cur = r0;
-        continue;
-      } else if (h1) {
-        cur = r1;
-        continue;
-      }
-    } else if (!inside) { /* top-level leaf: enter the instance */
+    const bool inner = cur >= 0;
+    if (!inner && !inside) { /* top-level leaf: enter the instance */
       const DevInstance &I = sc.instances[leaf_first(cur)];
       if (!I.identity) {
         ro = xform_point(I.inv, o);
         rd = xform_dir(I.inv, d);
-        ix = safe_rcp(rd.x), iy = safe_rcp(rd.y), iz = safe_rcp(rd.z);
+        sr.set(ro, rd);
       }
       prim_base = I.prim_offset;
       inst_in = leaf_first(cur);
@@ -461,36 +447,26 @@ NB_D TraceResult trace_closest_tl(const DevScene &sc, V3 o, V3 d, uint64_t *node
       if (sp < kTraversalStack) stack[sp++] = kLeaveInstance;
       cur = (int32_t)sc.blas_root[I.mesh];
       continue;
+    }
+    const Rec q = load_rec(inner ? sc.nodes + 4 * (size_t)(uint32_t)cur : sc.tris + kTriStride * (size_t)leaf_first(cur));
+    if (inner) {
+      nv++;
+      if (visit_inner(q, sr, tmax, stack, sp, cur)) continue;
     } else { /* bottom-level leaf: object-space triangles, mesh-local ids */
-#if NB_LEAF_STEP
-      if (lk >= le) {
-        lk = leaf_first(cur);
-        le = lk + leaf_count(cur);
+      tt++;
+      float ht, hu, hv;
+      if (visit_tri(q, ro, rd, tmax, ht, hu, hv)) {
+        tmax = ht;
+        r.prim = (int32_t)(prim_base + __float_as_uint(q.q0.w));
+        r.inst = inst_in;
+        r.t = ht;
+        r.u = hu;
+        r.v = hv;
       }
-      {
-        const uint32_t k = lk++;
-#else
-      const uint32_t first = leaf_first(cur), count = leaf_count(cur);
-      for (uint32_t k = first; k < first + count; k++) {
-#endif
-        const float4 t0 = __ldg(&sc.tris[3 * k + 0]);
-        const float4 t1 = __ldg(&sc.tris[3 * k + 1]);
-        const float4 t2 = __ldg(&sc.tris[3 * k + 2]);
-        tt++;
-        float ht, hu, hv;
-        if (mt_hit(ro, rd, V3{t0.x, t0.y, t0.z}, V3{t1.x, t1.y, t1.z}, V3{t2.x, t2.y, t2.z}, kRayTNear, tmax, ht, hu,
-                   hv)) {
-          tmax = ht;
-          r.prim = (int32_t)(prim_base + (uint32_t)__float_as_int(t0.w));
-          r.inst = inst_in;
-          r.t = ht;
-          r.u = hu;
-          r.v = hv;
-        }
+      if ((~cur & 15) != 0) {
+        cur -= 15;
+        continue;
       }
-#if NB_LEAF_STEP
-      if (lk < le) continue;
-#endif
     }
     /* pop; the marker returns the walk to the top level and the world ray */
     for (;;) {
@@ -504,7 +480,7 @@ NB_D TraceResult trace_closest_tl(const DevScene &sc, V3 o, V3 d, uint64_t *node
       inside = false;
       ro = o;
       rd = d;
-      ix = safe_rcp(d.x), iy = safe_rcp(d.y), iz = safe_rcp(d.z);
+      sr.set(o, d);
     }
   }
 }
