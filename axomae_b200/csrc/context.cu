@@ -761,8 +761,6 @@ nova_b200_status nova_b200_destroy(nova_b200_ctx *c) {
   cudaFree(c->d_persist);
   if (c->h_cancel_map) cudaFreeHost(const_cast<int *>(c->h_cancel_map));
   if (c->h_wave) cudaFreeHost(c->h_wave);
-  for (cudaGraphExec_t g : c->graph_exec)
-    if (g) cudaGraphExecDestroy(g);
   for (cudaEvent_t e : c->ev_done)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : c->ev_wave)

@@ -11,7 +11,7 @@
  *              atomics; after the last allowed scatter the spawned direction looks up the
  *              environment directly (the reference traces that ray but discards the hit,
  *              Integrator.cpp:94-98)
- *   k_wave_end advances the device-side wave counters
+ *   k_finish   once every path has started and few are left: the rest of each path in one thread
  *   k_resolve  per pixel, adds the per-path radiance of the call's samples to the running sum in
  *              sample order and writes sum / samples (writeFramebuffer, api/engine.cpp:351-363)
  *
@@ -23,14 +23,11 @@
  * and each pixel's samples are added in sample order, so a frame rendered in a batch equals the
  * same frame rendered alone, bit for bit.
  *
- * Wave loop: the counters (active paths, next path, hits, survivors) live on the device and the
- * kernels read device-resident counts, so the host never waits between waves.  Waves are enqueued
- * in groups of four, two groups in flight: while the GPU runs one group the host reads the
- * previous group's counters (pinned memory, event-synchronised) and enqueues the next, so the GPU
- * does not wait for the host; a group issued after the last path finished finds empty queues and
- * returns at once.  A single-frame chunk launches its kernels directly; a batch chunk replays each
- * slot's group from a CUDA graph (captured once per job table, with event-record nodes timing
- * every trace and shade kernel).
+ * Wave loop: the counters (waiting rays, next path, hits) live on the device in a ring of wave entries
+ * and the kernels read their counts there, so a wave is enqueued while the one before it runs: the host
+ * reads a finished wave's counters (pinned memory, event-synchronised), which bound the rays of the
+ * waves after it, and sizes the next launches by them.  The job table is a kernel parameter, so a chunk
+ * needs no set-up: 32 KB of it cost a launch less than a graph of four waves per chunk did to capture.
  *
  * The recursive estimator e_0 + c_0 (e_1 + c_1 (... env)) is evaluated forward as
  * sum_k beta_k e_k + beta_K env with beta_k = c_0 ... c_{k-1}; a path whose result is not finite
@@ -59,7 +56,6 @@ constexpr uint32_t kQueueCapDefault = 1u << 23; /* rays per wave unless tuned */
 constexpr size_t kRadianceCapBytes = 4ull << 30;
 constexpr unsigned kRRDimBase = 200; /* Russian roulette decisions use Sobol dimension 200 + bounce */
 constexpr int kMaxDepth = 48;        /* 2 + 4 (depth + 1) Sobol dimensions must stay below 200 */
-constexpr int kWavesPerGraph = 4;    /* even: the queues end each graph launch where they started */
 
 struct RenderParams {
   int32_t W, H;
@@ -82,17 +78,25 @@ struct Job {
   uint32_t n_paths;
 };
 
-struct WaveCounters {
-  uint32_t n_active; /* rays waiting in the input queue */
+/* One wave's counters.  Wave k uses ring entry k & 3: its kernels read entry k, append survivors to
+ * entry k + 1 and clear entry k + 2, so no kernel between waves has to advance them. */
+struct WaveState {
+  uint32_t n_active; /* rays waiting in the wave's input queue */
   uint32_t next;     /* next path id to start */
-  uint32_t total;    /* paths in the chunk */
-  uint32_t cap;      /* queue capacity */
-  uint32_t hit_count, out_count;
-  uint32_t hit_back; /* NB_HIT_CLASSES: hits of transmissive materials, from the end of the hit list */
-  uint32_t done;
-  uint32_t waves; /* waves that did work */
+  uint32_t hit_count;
+  uint32_t hit_back;   /* hits of transmissive materials, from the end of the hit list */
   uint32_t trace_next; /* next queued ray handed out by the persistent trace kernel */
   uint32_t shade_next; /* next hit handed out in the persistent wavefront */
+};
+constexpr uint32_t kWaveRing = 4;
+
+struct WaveCounters {
+  WaveState w[kWaveRing];
+  uint32_t total; /* paths in the chunk */
+  uint32_t cap;   /* queue capacity */
+  uint32_t waves; /* waves that did work */
+  uint32_t finish_waves; /* most segments a path took in k_finish: the waves it stands for */
+  uint32_t done;         /* persistent wavefront: every path has ended */
   /* device status of the whole loop (never reset between waves): path radiance values that were not
    * finite and were written as 0 (the reference's DENAN, Integrator.cpp:92), and hits whose
    * primitive, instance or material id is out of range (the path ends black, the render fails) */
@@ -133,8 +137,28 @@ struct Queue {
   float4 *o, *d, *beta;
 };
 
-__device__ __forceinline__ uint32_t wave_new(const WaveCounters &wc) {
-  return min(wc.cap - wc.n_active, wc.total - wc.next);
+/* New paths that start in the wave of entry `ws`, and the wave's rays. */
+__device__ __forceinline__ uint32_t wave_new(const WaveCounters &wc, const WaveState &ws) {
+  return min(wc.cap - ws.n_active, wc.total - ws.next);
+}
+__device__ __forceinline__ uint32_t wave_rays(const WaveCounters &wc, const WaveState &ws) {
+  return ws.n_active + wave_new(wc, ws);
+}
+__device__ __forceinline__ WaveState &wave_at(WaveCounters *wc, uint32_t k) { return wc->w[k & (kWaveRing - 1u)]; }
+
+/* The next wave's first path and the wave statistics, by one thread of wave k's trace pass. */
+__device__ __forceinline__ void advance_wave(WaveCounters *wc, uint32_t k) {
+  const WaveState &ws = wave_at(wc, k);
+  const uint32_t n_new = wave_new(*wc, ws), n = ws.n_active + n_new;
+  wave_at(wc, k + 1).next = ws.next + n_new;
+  wc->traced += n;
+  if (n) wc->waves++;
+}
+
+/* Entry k + 2 cleared for its wave, by one thread of wave k's shading pass. */
+__device__ __forceinline__ void clear_wave(WaveCounters *wc, uint32_t k) {
+  WaveState &ws = wave_at(wc, k + 2);
+  ws.n_active = ws.hit_count = ws.hit_back = ws.trace_next = ws.shade_next = 0;
 }
 
 constexpr uint32_t kTileW = 8, kTileH = 4; /* default pixel tile: one warp of camera rays per tile */
@@ -225,12 +249,12 @@ __device__ __forceinline__ void refill_one(const Queue &q, uint32_t next, uint32
 }
 
 template <class JS>
-__global__ void __launch_bounds__(256) k_refill(Queue q, const WaveCounters *wcp, float4 *L,
+__global__ void __launch_bounds__(256) k_refill(Queue q, WaveCounters *wcp, uint32_t wave, float4 *L,
                                                 const __grid_constant__ JS js) {
-  const WaveCounters wc = *wcp;
-  const uint32_t n_new = wave_new(wc);
+  const WaveState ws = wave_at(wcp, wave);
+  const uint32_t n_new = wave_new(*wcp, ws);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += gridDim.x * blockDim.x)
-    refill_one(q, wc.next, wc.n_active, L, js, i);
+    refill_one(q, ws.next, ws.n_active, L, js, i);
 }
 
 /* Non-finite radiance becomes 0 (DENAN), counted in *nonfinite (rare: a plain atomic). */
@@ -301,36 +325,33 @@ __device__ __forceinline__ unsigned warp_append(bool flag, unsigned *counter) {
 template <int WIDTH>
 constexpr int kTraceBlocks = WIDTH == 1 ? 9 : 10;
 
-/* NB_HIT_CLASSES=1: the hit list holds non-transmissive hits from its front and transmissive ones
- * from its back (k_shade reads both ranges), so shading warps mostly run one lobe family: the
- * dielectric lobe's refraction code or the reflective lobes'.  The class is the instance's (its
- * material's eta and k, NovaMaterials.h:118-121), read next to the identity flag the traversal
- * already loaded.  On the 32-job batch k_shade went from 107.3 to 80.9 ms per step (films
- * bit-identical); only the order in which hits are shaded changes.  A third list for fully metal
- * materials measured equal (shading -0.6 %, the third append +0.4 % in k_trace). */
-#ifndef NB_HIT_CLASSES
-#define NB_HIT_CLASSES 1
-#endif
+/* The hit list holds non-transmissive hits from its front and transmissive ones from its back (k_shade
+ * reads both ranges), so shading warps mostly run one lobe family: the dielectric lobe's refraction
+ * code or the reflective lobes'.  The class is the instance's (its material's eta and k,
+ * NovaMaterials.h:118-121).  On 32 frames k_shade went from 107.3 to 80.9 ms (films bit-identical);
+ * only the order in which hits are shaded changes.  A third list for fully metal materials measured
+ * equal (shading -0.6 %, the third append +0.4 % in k_trace). */
 
 /* The closest-hit pass for one warp's lanes (ray i of n queued; the warp's lanes call together: the
  * hit append is a warp ballot). */
 template <int WIDTH, class JS, bool ADJ, bool COUNT, bool P>
-__device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, float4 *hits, uint2 *hit_slot,
-                                           float4 *L, const JS &js, uint32_t i, uint32_t n,
-                                           const uint32_t *order = nullptr) {
+__device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, WaveState &ws, float4 *hits,
+                                           uint2 *hit_slot, float4 *L, const JS &js, uint32_t i, uint32_t n) {
   {
     bool is_hit = false, back = false;
     TraceResult r{-1, 0.f, 0.f, 0.f, 0u};
     uint64_t nv = 0, tt = 0;
     if (i < n) {
-      if (order) i = order[i]; /* the queue slot this lane traces (k_order_rays) */
       const float4 o = ldq<P>(&q.o[i]), d = ldq<P>(&q.d[i]);
       const DevScene &sc = js.at(__float_as_uint(d.w) >> 8).sc;
-      r = trace_closest_w<WIDTH>(sc, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, COUNT ? &nv : nullptr,
-                                 COUNT ? &tt : nullptr);
+      if constexpr (P)
+        r = walk<WIDTH>(sc, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z});
+      else
+        r = trace_closest_w<WIDTH>(sc, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, COUNT ? &nv : nullptr,
+                                   COUNT ? &tt : nullptr);
       if (r.prim >= 0) {
         is_hit = true;
-        if constexpr (NB_HIT_CLASSES && !COUNT && !P) back = sc.instances[r.inst].lobe_class != 0u;
+        if constexpr (!COUNT && !P) back = sc.instances[r.inst].lobe_class != 0u;
       } else if (!ADJ) { /* a replayed path's radiance is already known */
         const float4 b4 = ldq<P>(&q.beta[i]);
         const V4 e = env_sample(sc, V3{d.x, d.y, d.z});
@@ -351,14 +372,14 @@ __device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, fl
       }
     }
     uint32_t slot;
-    if constexpr (NB_HIT_CLASSES && !COUNT && !P) {
+    if constexpr (!COUNT && !P) {
       /* transmissive hits go to the end of the list, the others to the front, so the shading warps
        * mostly take one lobe family (BSDF.h:69-79) */
-      const unsigned f = warp_append(is_hit && !back, &wcp->hit_count);
-      const unsigned b = warp_append(back, &wcp->hit_back);
+      const unsigned f = warp_append(is_hit && !back, &ws.hit_count);
+      const unsigned b = warp_append(back, &ws.hit_back);
       slot = back ? wcp->cap - 1u - b : f;
     } else {
-      slot = warp_append(is_hit, &wcp->hit_count);
+      slot = warp_append(is_hit, &ws.hit_count);
     }
     if (is_hit) {
       hits[slot] = make_float4(r.t, r.u, r.v, __int_as_float(r.prim));
@@ -369,73 +390,14 @@ __device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, fl
 
 template <int WIDTH, class JS, bool ADJ = false, bool COUNT = false>
 __global__ void __launch_bounds__(128, kTraceBlocks<WIDTH>)
-    k_trace(Queue q, WaveCounters *wcp, float4 *hits, uint2 *hit_slot, float4 *L,
-            const __grid_constant__ JS js, const uint32_t *order = nullptr) {
-  const uint32_t n = wcp->n_active + wave_new(*wcp);
+    k_trace(Queue q, WaveCounters *wcp, uint32_t wave, float4 *hits, uint2 *hit_slot, float4 *L,
+            const __grid_constant__ JS js) {
+  WaveState &ws = wave_at(wcp, wave);
+  const uint32_t n = wave_rays(*wcp, ws);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if ((i & ~31u) >= n) return; /* whole warps leave together (the append below is a warp ballot) */
-  trace_warp<WIDTH, JS, ADJ, COUNT, false>(q, wcp, hits, hit_slot, L, js, i, n, order);
-}
-
-/* Ray ordering before the trace (NB_RAY_ORDER = window of queue slots, 0 = off): each window of
- * consecutive slots, whose rays come from neighbouring pixel tiles, is counting-sorted by direction
- * (8 x 8 octahedral bins), and k_trace's warps take the window's rays in that order, so a warp's
- * rays start out alike.  Only the order in which rays are traced and appended changes; a path's
- * result does not depend on it. */
-#ifndef NB_RAY_ORDER
-#define NB_RAY_ORDER 0
-#endif
-constexpr int kOrderThreads = 1024;
-
-__device__ __forceinline__ uint32_t direction_bin(float4 d) {
-  const float s = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
-  float x = d.x / s, y = d.y / s;
-  if (d.z < 0.f) {
-    const float ax = fabsf(x), ay = fabsf(y);
-    x = copysignf(1.f - ay, x);
-    y = copysignf(1.f - ax, y);
-  }
-  const int bx = min(7, max(0, (int)((x + 1.f) * 4.f))), by = min(7, max(0, (int)((y + 1.f) * 4.f)));
-  return (uint32_t)(bx + 8 * by);
-}
-
-template <int WINDOW>
-__global__ void __launch_bounds__(kOrderThreads) k_order_rays(Queue q, const WaveCounters *wcp, uint32_t *order) {
-  constexpr int kPer = WINDOW / kOrderThreads;
-  __shared__ uint32_t s_bin[64];
-  const uint32_t n = wcp->n_active + wave_new(*wcp);
-  const uint32_t start = blockIdx.x * (uint32_t)WINDOW;
-  if (start >= n) return;
-  if (threadIdx.x < 64) s_bin[threadIdx.x] = 0;
-  __syncthreads();
-  uint32_t key[kPer];
-#pragma unroll
-  for (int k = 0; k < kPer; k++) {
-    const uint32_t slot = start + (uint32_t)k * kOrderThreads + threadIdx.x;
-    key[k] = 64u;
-    if (slot < n) {
-      key[k] = direction_bin(q.d[slot]);
-      atomicAdd(&s_bin[key[k]], 1u);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) { /* exclusive scan of the 64 bins by one warp, two bins a lane */
-    const uint32_t a = s_bin[2 * threadIdx.x], b = s_bin[2 * threadIdx.x + 1];
-    uint32_t x = a + b;
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-      if ((int)threadIdx.x >= off) x += y;
-    }
-    const uint32_t excl = x - a - b;
-    s_bin[2 * threadIdx.x] = excl;
-    s_bin[2 * threadIdx.x + 1] = excl + a;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kPer; k++) {
-    const uint32_t slot = start + (uint32_t)k * kOrderThreads + threadIdx.x;
-    if (key[k] < 64u) order[start + atomicAdd(&s_bin[key[k]], 1u)] = slot;
-  }
+  if (i == 0) advance_wave(wcp, wave);
+  if ((i & ~31u) >= n) return; /* whole warps leave together (the append is a warp ballot) */
+  trace_warp<WIDTH, JS, ADJ, COUNT, false>(q, wcp, ws, hits, hit_slot, L, js, i, n);
 }
 
 /* Persistent variant of k_trace (binary BVH): a fixed grid of warps hands out the queued rays with
@@ -461,10 +423,12 @@ constexpr int kDynSteps = NB_DYN_STEPS;
 constexpr int kRefillLanes = 8;
 
 template <class JS>
-__global__ void __launch_bounds__(128, NB_DYN_MIN_BLOCKS) k_trace_dyn(Queue q, WaveCounters *wcp, float4 *hits,
-                                                                      uint2 *hit_slot, float4 *L,
+__global__ void __launch_bounds__(128, NB_DYN_MIN_BLOCKS) k_trace_dyn(Queue q, WaveCounters *wcp, uint32_t wave,
+                                                                      float4 *hits, uint2 *hit_slot, float4 *L,
                                                                       const __grid_constant__ JS js) {
-  const uint32_t n = wcp->n_active + wave_new(*wcp);
+  WaveState &ws_ = wave_at(wcp, wave);
+  const uint32_t n = wave_rays(*wcp, ws_);
+  if (blockIdx.x == 0 && threadIdx.x == 0) advance_wave(wcp, wave);
   const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
   Walk2 w;
   WalkScene ws{nullptr, nullptr, nullptr};
@@ -478,7 +442,7 @@ __global__ void __launch_bounds__(128, NB_DYN_MIN_BLOCKS) k_trace_dyn(Queue q, W
     if (need) {
       const int leader = __ffs(need) - 1;
       uint32_t base = 0;
-      if ((int)lane == leader) base = atomicAdd(&wcp->trace_next, (unsigned)__popc(need));
+      if ((int)lane == leader) base = atomicAdd(&ws_.trace_next, (unsigned)__popc(need));
       base = __shfl_sync(full, base, leader);
       if (idle) {
         const uint32_t i = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
@@ -510,7 +474,7 @@ __global__ void __launch_bounds__(128, NB_DYN_MIN_BLOCKS) k_trace_dyn(Queue q, W
                   &wcp->nonfinite);
     }
     if (__ballot_sync(full, fin)) {
-      const unsigned slot = warp_append(is_hit, &wcp->hit_count);
+      const unsigned slot = warp_append(is_hit, &ws_.hit_count);
       if (is_hit) {
         hits[slot] = make_float4(w.r.t, w.r.u, w.r.v, __int_as_float(w.r.prim));
         hit_slot[slot] = make_uint2((uint32_t)ray, w.r.inst);
@@ -520,167 +484,115 @@ __global__ void __launch_bounds__(128, NB_DYN_MIN_BLOCKS) k_trace_dyn(Queue q, W
   }
 }
 
-/* The shading pass for one warp's lanes (hit i of n; the warp's lanes call together: the continuation
- * append is a warp ballot). */
+/* Shades one path at its hit (t, u, v, prim) on instance `inst`: true when it goes on, with the spawned
+ * ray in o4, d4, b4; else its radiance has been written. */
 template <class JS, bool P>
-__device__ __forceinline__ void shade_warp(const Queue &in, const Queue &out, WaveCounters *wcp, const float4 *hits,
-                                           const uint2 *hit_slot, float4 *L, const JS &js, uint32_t i, uint32_t n) {
-  {
-    bool enq = false;
-    float4 no{}, nd{}, nbeta{};
-    if (i < n) {
-      const uint2 hs = ldq<P>(&hit_slot[i]);
-      const uint32_t slot_in = hs.x, inst = hs.y;
-      const float4 o4 = ldq<P>(&in.o[slot_in]), d4 = ldq<P>(&in.d[slot_in]), b4 = ldq<P>(&in.beta[slot_in]),
-                   h = ldq<P>(&hits[i]);
-      const uint32_t g = __float_as_uint(o4.w);
-      const uint32_t tag = __float_as_uint(d4.w);
-      const int bounce = (int)(tag & 0xffu);
-      const Job &J = js.at(tag >> 8);
-      const DevScene &sc = J.sc;
-      const RenderParams &rp = J.rp;
-      const uint32_t index = __float_as_uint(b4.w); /* the path's Sobol index, set by k_refill */
-      const V3 ro{o4.x, o4.y, o4.z}, rd{d4.x, d4.y, d4.z};
-      V3 beta{b4.x, b4.y, b4.z};
-      const int prim = __float_as_int(h.w);
-      bool done = false;
-      float4 result = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!hit_ids_valid(sc, prim, inst)) {
-        atomicAdd(&wcp->bad_index, 1u);
-        L[g] = make_float4(0.f, 0.f, 0.f, 0.f);
-        goto append;
-      }
-      {
-      const DevInstance &I = sc.instances[inst];
-      const HitRecord hr = make_record(sc, ro, rd, I, (uint32_t)prim - I.prim_offset, h.x, h.y, h.z);
-      const ScatterResult sr = scatter(sc, rd, hr, sc.materials[I.material], index, 2u + 4u * (unsigned)bounce, rp.seed,
-                                       (uint32_t)prim, I.material);
-      /* a failed scatter returns black, emission included (Integrator.cpp:73-79) */
-      if (sr.valid && sc.has_emissive && any_nonzero(sr.emissive)) {
-        const V3 em = beta * sr.emissive;
-        const float4 acc = ldq<P>(&L[g]);
-        L[g] = make_float4(acc.x + em.x, acc.y + em.y, acc.z + em.z, acc.w);
-      }
-      if (!sr.valid) {
-        result = make_float4(0.f, 0.f, 0.f, (float)bounce);
-        done = true;
+__device__ __forceinline__ bool shade_path(float4 &o4, float4 &d4, float4 &b4, const float4 &h, uint32_t inst,
+                                           WaveCounters *wcp, float4 *L, const JS &js) {
+  const uint32_t g = __float_as_uint(o4.w);
+  const uint32_t tag = __float_as_uint(d4.w);
+  const int bounce = (int)(tag & 0xffu);
+  const Job &J = js.at(tag >> 8);
+  const DevScene &sc = J.sc;
+  const RenderParams &rp = J.rp;
+  const uint32_t index = __float_as_uint(b4.w); /* the path's Sobol index, set by k_refill */
+  const V3 ro{o4.x, o4.y, o4.z}, rd{d4.x, d4.y, d4.z};
+  V3 beta{b4.x, b4.y, b4.z};
+  const int prim = __float_as_int(h.w);
+  if (!hit_ids_valid(sc, prim, inst)) {
+    atomicAdd(&wcp->bad_index, 1u);
+    L[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return false;
+  }
+  const DevInstance &I = sc.instances[inst];
+  const HitRecord hr = make_record(sc, ro, rd, I, (uint32_t)prim - I.prim_offset, h.x, h.y, h.z);
+  const ScatterResult sr = scatter(sc, rd, hr, sc.materials[I.material], index, 2u + 4u * (unsigned)bounce, rp.seed,
+                                   (uint32_t)prim, I.material);
+  /* a failed scatter returns black, emission included (Integrator.cpp:73-79) */
+  if (sr.valid && sc.has_emissive && any_nonzero(sr.emissive)) {
+    const V3 em = beta * sr.emissive;
+    const float4 acc = ldq<P>(&L[g]);
+    L[g] = make_float4(acc.x + em.x, acc.y + em.y, acc.z + em.z, acc.w);
+  }
+  float4 result = make_float4(0.f, 0.f, 0.f, (float)bounce);
+  if (sr.valid) {
+    V3 c = sr.weight;
+    bool alive = true;
+    if (rp.rr_start >= 0 && bounce >= rp.rr_start) {
+      const V3 nbt = beta * c;
+      const float q = fmin_std(1.f, fmax_std(0.05f, fmax_std(nbt.x, fmax_std(nbt.y, nbt.z))));
+      const float urr = sobol_sample(sc.sobol_dv, index, kRRDimBase + (unsigned)bounce, rp.seed);
+      if (!(urr < q)) {
+        alive = false;
+        result = make_float4(0.f, 0.f, 0.f, (float)bounce + 1.f);
       } else {
-        V3 c = sr.weight;
-        bool alive = true;
-        if (rp.rr_start >= 0 && bounce >= rp.rr_start) {
-          const V3 nbt = beta * c;
-          const float q = fmin_std(1.f, fmax_std(0.05f, fmax_std(nbt.x, fmax_std(nbt.y, nbt.z))));
-          const float urr = sobol_sample(sc.sobol_dv, index, kRRDimBase + (unsigned)bounce, rp.seed);
-          if (!(urr < q)) {
-            alive = false;
-            result = make_float4(0.f, 0.f, 0.f, (float)bounce + 1.f);
-            done = true;
-          } else {
-            c = c / q;
-          }
-        }
-        if (alive) {
-          beta = beta * c;
-          const float eps = 1e-3f; /* Ray::spawn, ray/Ray.h:22-27 */
-          const V3 nd3 = normalize(sr.wi);
-          const V3 no3 = hr.position + hr.ng * (eps + eps * fsign(dot(hr.ng, sr.wi)));
-          if (bounce + 1 > rp.max_depth) {
-            const V4 e = env_sample(sc, nd3);
-            result = finite_or_zero(beta * V3{e.x, e.y, e.z}, (float)bounce + 1.f + e.w, &wcp->nonfinite);
-            done = true;
-          } else {
-            enq = true;
-            no = make_float4(no3.x, no3.y, no3.z, o4.w);
-            nd = make_float4(nd3.x, nd3.y, nd3.z, __uint_as_float(tag + 1u));
-            nbeta = make_float4(beta.x, beta.y, beta.z, b4.w);
-          }
-        }
-      }
-      if (done) finish_path<P>(sc, L, g, result, &wcp->nonfinite);
+        c = c / q;
       }
     }
-  append:
-    const unsigned slot = warp_append(enq, &wcp->out_count);
-    if (enq) {
-      out.o[slot] = no;
-      out.d[slot] = nd;
-      out.beta[slot] = nbeta;
+    if (alive) {
+      beta = beta * c;
+      const float eps = 1e-3f; /* Ray::spawn, ray/Ray.h:22-27 */
+      const V3 nd3 = normalize(sr.wi);
+      const V3 no3 = hr.position + hr.ng * (eps + eps * fsign(dot(hr.ng, sr.wi)));
+      if (bounce + 1 > rp.max_depth) {
+        const V4 e = env_sample(sc, nd3);
+        result = finite_or_zero(beta * V3{e.x, e.y, e.z}, (float)bounce + 1.f + e.w, &wcp->nonfinite);
+      } else {
+        o4 = make_float4(no3.x, no3.y, no3.z, o4.w);
+        d4 = make_float4(nd3.x, nd3.y, nd3.z, __uint_as_float(tag + 1u));
+        b4 = make_float4(beta.x, beta.y, beta.z, b4.w);
+        return true;
+      }
     }
+  }
+  finish_path<P>(sc, L, g, result, &wcp->nonfinite);
+  return false;
+}
+
+/* The shading pass for one warp's lanes (hit i, when the lane has one; the warp's lanes call together:
+ * the continuation append is a warp ballot). */
+template <class JS, bool P>
+__device__ __forceinline__ void shade_warp(const Queue &in, const Queue &out, WaveCounters *wcp, unsigned *out_count,
+                                           const float4 *hits, const uint2 *hit_slot, float4 *L, const JS &js,
+                                           uint32_t i, bool valid) {
+  bool enq = false;
+  float4 o4{}, d4{}, b4{};
+  if (valid) {
+    const uint2 hs = ldq<P>(&hit_slot[i]);
+    o4 = ldq<P>(&in.o[hs.x]), d4 = ldq<P>(&in.d[hs.x]), b4 = ldq<P>(&in.beta[hs.x]);
+    enq = shade_path<JS, P>(o4, d4, b4, ldq<P>(&hits[i]), hs.y, wcp, L, js);
+  }
+  const unsigned slot = warp_append(enq, out_count);
+  if (enq) {
+    out.o[slot] = o4;
+    out.d[slot] = d4;
+    out.beta[slot] = b4;
   }
 }
 
-/* Lobe class of hit i, the key k_shade groups a block's hits by (BSDF.h:69-79 picks the lobe from
- * the material's transmission and metallic inputs): 0 diffuse-only material, 1 a material with a
- * metallic/roughness texture, 2 a transmissive one (eta set, no absorption), 3 no hit / bad index. */
-template <class JS>
-__device__ __forceinline__ uint32_t lobe_class(const Queue &in, const float4 *hits, const uint2 *hit_slot,
-                                               const JS &js, uint32_t i, uint32_t n) {
-  if (i >= n) return 3u;
-  const uint2 hs = hit_slot[i];
-  const uint32_t tag = __float_as_uint(in.d[hs.x].w), inst = hs.y;
-  const DevScene &sc = js.at(tag >> 8).sc;
-  const int prim = __float_as_int(hits[i].w);
-  if (!hit_ids_valid(sc, prim, inst)) return 3u;
-  const DevMaterial &m = sc.materials[sc.instances[inst].material];
-  const bool eta = m.eta[0] != 0.f || m.eta[1] != 0.f || m.eta[2] != 0.f;
-  const bool k = m.k[0] != 0.f || m.k[1] != 0.f || m.k[2] != 0.f;
-  return (eta && !k) ? 2u : (m.metallic >= 0 ? 1u : 0u);
-}
-
-#ifndef NB_SHADE_SORT
-#define NB_SHADE_SORT 0
-#endif
-static_assert(!(NB_HIT_CLASSES && NB_SHADE_SORT), "one hit ordering at a time");
-
 /* Resident blocks of 128 per SM that k_shade is compiled for.  With hits of one lobe family per
- * warp (NB_HIT_CLASSES), 8 blocks (64 registers) are best on the 32-job batch: 79.5 ms per step,
- * against 79.9 at 9, 80.7 at 10 (48 registers, more spills) and 81.4 at 12; before the split 10
- * blocks led (107.5 ms against 108.6 at 8), and 8 also suits the heightfield (11.7 against 12.1). */
+ * warp, 8 blocks (64 registers) are best on 32 frames: 79.5 ms per step, against 79.9 at 9, 80.7 at 10
+ * (48 registers, more spills) and 81.4 at 12; 8 also suits the heightfield (11.7 against 12.1). */
 #ifndef NB_SHADE_MIN_BLOCKS
 #define NB_SHADE_MIN_BLOCKS 8
 #endif
 
+/* Hit t of a wave: of the front range, or of the back range counted from the end of the list. */
+__device__ __forceinline__ uint32_t hit_index(uint32_t t, uint32_t front, uint32_t cap) {
+  return t < front ? t : cap - 1u - (t - front);
+}
+
 template <class JS>
-__global__ void __launch_bounds__(128, NB_SHADE_MIN_BLOCKS) k_shade(Queue in, Queue out, WaveCounters *wcp, const float4 *hits,
-                                               const uint2 *hit_slot, float4 *L, const __grid_constant__ JS js) {
-  const uint32_t n = wcp->hit_count;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-#if NB_SHADE_SORT
-  /* The block's 128 hits are permuted so that each lobe class runs contiguously (a counting sort of
-   * four keys with warp ballots): warps then take one lobe's code path.  Only the order of the
-   * continuation rays changes, never a path's result. */
-  if (blockIdx.x * blockDim.x >= n) return; /* whole blocks leave together (barriers below) */
-  __shared__ uint32_t s_cnt[4][4];
-  __shared__ uint8_t s_perm[128];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t cls = lobe_class(in, hits, hit_slot, js, i, n);
-  const unsigned mine = __ballot_sync(0xffffffffu, cls == 0u) * (cls == 0u) |
-                        __ballot_sync(0xffffffffu, cls == 1u) * (cls == 1u) |
-                        __ballot_sync(0xffffffffu, cls == 2u) * (cls == 2u) |
-                        __ballot_sync(0xffffffffu, cls == 3u) * (cls == 3u);
-  if (threadIdx.x < 16u) (&s_cnt[0][0])[threadIdx.x] = 0; /* blocks of fewer than 4 warps count 0 for the rest */
-  __syncthreads();
-  if (lane == (uint32_t)(__ffs(mine) - 1)) s_cnt[warp][cls] = (uint32_t)__popc(mine);
-  __syncthreads();
-  uint32_t pos = (uint32_t)__popc(mine & ((1u << lane) - 1u));
-  for (uint32_t c = 0; c < cls; c++)
-    pos += s_cnt[0][c] + s_cnt[1][c] + s_cnt[2][c] + s_cnt[3][c];
-  for (uint32_t w = 0; w < warp; w++) pos += s_cnt[w][cls];
-  s_perm[pos] = (uint8_t)threadIdx.x;
-  __syncthreads();
-  i = blockIdx.x * blockDim.x + s_perm[threadIdx.x];
-  if (__all_sync(0xffffffffu, i >= n)) return;
-#elif NB_HIT_CLASSES
-  const uint32_t nf = n, nb = wcp->hit_back, cap = wcp->cap;
-  if ((i & ~31u) >= nf + nb) return;
-  /* hit i of the front range, or of the back range counted from the end of the list */
-  const uint32_t h = i < nf ? i : (i < nf + nb ? cap - 1u - (i - nf) : 0u);
-  shade_warp<JS, false>(in, out, wcp, hits, hit_slot, L, js, h, i < nf + nb ? 0xffffffffu : 0u);
-  return;
-#else
-  if ((i & ~31u) >= n) return;
-#endif
-  shade_warp<JS, false>(in, out, wcp, hits, hit_slot, L, js, i, n);
+__global__ void __launch_bounds__(128, NB_SHADE_MIN_BLOCKS)
+    k_shade(Queue in, Queue out, WaveCounters *wcp, uint32_t wave, const float4 *hits, const uint2 *hit_slot, float4 *L,
+            const __grid_constant__ JS js) {
+  const WaveState &ws = wave_at(wcp, wave);
+  const uint32_t nf = ws.hit_count, n = nf + ws.hit_back, cap = wcp->cap;
+  unsigned *out_count = &wave_at(wcp, wave + 1).n_active;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) clear_wave(wcp, wave);
+  if ((t & ~31u) >= n) return;
+  shade_warp<JS, false>(in, out, wcp, out_count, hits, hit_slot, L, js, hit_index(t, nf, cap), t < n);
 }
 
 /* ---------------------------------------------------------------- replay adjoint
@@ -736,14 +648,15 @@ __device__ __forceinline__ void warp_add_by_key(bool active, uint32_t key, const
 }
 
 template <class JS>
-__global__ void __launch_bounds__(256) k_refill_adj(Queue q, AdjQueue a, const WaveCounters *wcp, const float4 *L,
-                                                    const float4 *d_image, const __grid_constant__ JS js) {
-  const WaveCounters wc = *wcp;
-  const uint32_t n_new = wave_new(wc);
+__global__ void __launch_bounds__(256) k_refill_adj(Queue q, AdjQueue a, WaveCounters *wcp, uint32_t wave,
+                                                    const float4 *L, const float4 *d_image,
+                                                    const __grid_constant__ JS js) {
+  const WaveState ws = wave_at(wcp, wave);
+  const uint32_t n_new = wave_new(*wcp, ws);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += gridDim.x * blockDim.x) {
-    const CameraPath c = camera_path(js, wc.next + i);
+    const CameraPath c = camera_path(js, ws.next + i);
     const RenderParams &rp = js.at(c.job).rp;
-    const uint32_t slot = wc.n_active + i;
+    const uint32_t slot = ws.n_active + i;
     q.o[slot] = make_float4(c.o.x, c.o.y, c.o.z, __uint_as_float(c.rslot));
     q.d[slot] = make_float4(c.d.x, c.d.y, c.d.z, __uint_as_float(c.job << 8));
     q.beta[slot] = make_float4(1.f, 1.f, 1.f, __uint_as_float(c.index));
@@ -757,118 +670,175 @@ __global__ void __launch_bounds__(256) k_refill_adj(Queue q, AdjQueue a, const W
   }
 }
 
+/* One vertex's terms of the gradients. */
+struct AdjTerms {
+  bool active;
+  uint32_t prim, mat;
+  float albedo[3], rough[1];
+};
+
+/* Replays one path's vertex at its hit: its gradient terms, and true when the path goes on, with the
+ * spawned ray in o4, d4, b4 and what it still gathers in rem. */
 template <class JS>
-__global__ void __launch_bounds__(128, 8) k_shade_adj(Queue in, Queue out, AdjQueue ain, AdjQueue aout,
-                                                      WaveCounters *wcp, const float4 *hits, const uint2 *hit_slot,
-                                                      float *g_alb, float *g_rough, const __grid_constant__ JS js) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-#if NB_HIT_CLASSES
-  /* the front range of the hit list, then its back range counted from the end (see k_shade) */
-  const uint32_t nf = wcp->hit_count, nb = wcp->hit_back, cap = wcp->cap;
-  if ((t & ~31u) >= nf + nb) return;
-  const bool valid = t < nf + nb;
-  const uint32_t i = t < nf ? t : (valid ? cap - 1u - (t - nf) : 0u);
-#else
-  const uint32_t n = wcp->hit_count;
-  if ((t & ~31u) >= n) return;
-  const bool valid = t < n;
-  const uint32_t i = t;
-#endif
-  bool enq = false, g_act = false;
-  float4 no{}, nd{}, nbeta{}, nrem{}, ndl{};
-  uint32_t g_prim = 0, g_mat = 0;
-  float va[3] = {0.f, 0.f, 0.f}, vr[1] = {0.f};
-  if (valid) {
-    const uint2 hs = hit_slot[i];
-    const uint32_t slot_in = hs.x, inst = hs.y;
-    const float4 o4 = in.o[slot_in], d4 = in.d[slot_in], b4 = in.beta[slot_in], h = hits[i];
-    const float4 r4 = ain.rem[slot_in], l4 = ain.dl[slot_in];
-    const uint32_t tag = __float_as_uint(d4.w);
-    const int bounce = (int)(tag & 0xffu);
-    const Job &J = js.at(tag >> 8);
-    const DevScene &sc = J.sc;
-    const RenderParams &rp = J.rp;
-    const uint32_t index = __float_as_uint(b4.w);
-    const V3 ro{o4.x, o4.y, o4.z}, rd{d4.x, d4.y, d4.z};
-    V3 beta{b4.x, b4.y, b4.z};
-    V3 rem{r4.x, r4.y, r4.z};
-    const V3 dl{l4.x, l4.y, l4.z};
-    const int prim = __float_as_int(h.w);
-    if (!hit_ids_valid(sc, prim, inst)) {
-      atomicAdd(&wcp->bad_index, 1u);
-      goto gather;
-    }
-    {
-    const DevInstance &I = sc.instances[inst];
-    const HitRecord hr = make_record(sc, ro, rd, I, (uint32_t)prim - I.prim_offset, h.x, h.y, h.z);
-    Scores scs;
-    const ScatterResult sr = scatter(sc, rd, hr, sc.materials[I.material], index, 2u + 4u * (unsigned)bounce, rp.seed,
-                                     (uint32_t)prim, I.material, &scs);
-    if (sr.valid && sc.has_emissive) rem = rem - beta * sr.emissive;
-    if (sr.valid) {
-      const V3 cw = dl * rem;
-      g_act = true;
-      g_prim = (uint32_t)prim;
-      g_mat = I.material;
-      va[0] = cw.x * scs.albedo.x;
-      va[1] = cw.y * scs.albedo.y;
-      va[2] = cw.z * scs.albedo.z;
-      const float gr = ((cw.x + cw.y) + cw.z) * scs.roughness;
-      vr[0] = isfinite(gr) ? gr : 0.f;
-      V3 c = sr.weight;
-      bool alive = true;
-      if (rp.rr_start >= 0 && bounce >= rp.rr_start) {
-        const V3 nbt = beta * c;
-        const float q = fmin_std(1.f, fmax_std(0.05f, fmax_std(nbt.x, fmax_std(nbt.y, nbt.z))));
-        const float urr = sobol_sample(sc.sobol_dv, index, kRRDimBase + (unsigned)bounce, rp.seed);
-        if (!(urr < q))
-          alive = false;
-        else
-          c = c / q;
-      }
-      if (alive && bounce + 1 <= rp.max_depth) {
-        beta = beta * c;
-        const float eps = 1e-3f;
-        const V3 nd3 = normalize(sr.wi);
-        const V3 no3 = hr.position + hr.ng * (eps + eps * fsign(dot(hr.ng, sr.wi)));
-        enq = true;
-        no = make_float4(no3.x, no3.y, no3.z, o4.w);
-        nd = make_float4(nd3.x, nd3.y, nd3.z, __uint_as_float(tag + 1u));
-        nbeta = make_float4(beta.x, beta.y, beta.z, b4.w);
-        nrem = make_float4(rem.x, rem.y, rem.z, 0.f);
-        ndl = l4;
-      }
-    }
-    }
+__device__ __forceinline__ bool shade_adj_path(float4 &o4, float4 &d4, float4 &b4, float4 &rem4, const float4 &l4,
+                                               const float4 &h, uint32_t inst, WaveCounters *wcp, const JS &js,
+                                               AdjTerms &g) {
+  const uint32_t tag = __float_as_uint(d4.w);
+  const int bounce = (int)(tag & 0xffu);
+  const Job &J = js.at(tag >> 8);
+  const DevScene &sc = J.sc;
+  const RenderParams &rp = J.rp;
+  const uint32_t index = __float_as_uint(b4.w);
+  const V3 ro{o4.x, o4.y, o4.z}, rd{d4.x, d4.y, d4.z};
+  V3 beta{b4.x, b4.y, b4.z};
+  V3 rem{rem4.x, rem4.y, rem4.z};
+  const V3 dl{l4.x, l4.y, l4.z};
+  const int prim = __float_as_int(h.w);
+  if (!hit_ids_valid(sc, prim, inst)) {
+    atomicAdd(&wcp->bad_index, 1u);
+    return false;
   }
-gather:
-  if (g_alb) warp_add_by_key<3>(g_act, g_prim, va, g_alb);
-  if (g_rough) warp_add_by_key<1>(g_act, g_mat, vr, g_rough);
-  const unsigned slot = warp_append(enq, &wcp->out_count);
+  const DevInstance &I = sc.instances[inst];
+  const HitRecord hr = make_record(sc, ro, rd, I, (uint32_t)prim - I.prim_offset, h.x, h.y, h.z);
+  Scores scs;
+  const ScatterResult sr = scatter(sc, rd, hr, sc.materials[I.material], index, 2u + 4u * (unsigned)bounce, rp.seed,
+                                   (uint32_t)prim, I.material, &scs);
+  if (!sr.valid) return false;
+  if (sc.has_emissive) rem = rem - beta * sr.emissive;
+  const V3 cw = dl * rem;
+  g.active = true;
+  g.prim = (uint32_t)prim;
+  g.mat = I.material;
+  g.albedo[0] = cw.x * scs.albedo.x;
+  g.albedo[1] = cw.y * scs.albedo.y;
+  g.albedo[2] = cw.z * scs.albedo.z;
+  const float gr = ((cw.x + cw.y) + cw.z) * scs.roughness;
+  g.rough[0] = isfinite(gr) ? gr : 0.f;
+  V3 c = sr.weight;
+  if (rp.rr_start >= 0 && bounce >= rp.rr_start) {
+    const V3 nbt = beta * c;
+    const float q = fmin_std(1.f, fmax_std(0.05f, fmax_std(nbt.x, fmax_std(nbt.y, nbt.z))));
+    const float urr = sobol_sample(sc.sobol_dv, index, kRRDimBase + (unsigned)bounce, rp.seed);
+    if (!(urr < q)) return false;
+    c = c / q;
+  }
+  if (bounce + 1 > rp.max_depth) return false;
+  beta = beta * c;
+  const float eps = 1e-3f;
+  const V3 nd3 = normalize(sr.wi);
+  const V3 no3 = hr.position + hr.ng * (eps + eps * fsign(dot(hr.ng, sr.wi)));
+  o4 = make_float4(no3.x, no3.y, no3.z, o4.w);
+  d4 = make_float4(nd3.x, nd3.y, nd3.z, __uint_as_float(tag + 1u));
+  b4 = make_float4(beta.x, beta.y, beta.z, b4.w);
+  rem4 = make_float4(rem.x, rem.y, rem.z, 0.f);
+  return true;
+}
+
+/* Adds the warp's terms to the gradients asked for (all 32 lanes call it). */
+__device__ __forceinline__ void add_terms(const AdjTerms &g, float *g_alb, float *g_rough) {
+  if (g_alb) warp_add_by_key<3>(g.active, g.prim, g.albedo, g_alb);
+  if (g_rough) warp_add_by_key<1>(g.active, g.mat, g.rough, g_rough);
+}
+
+template <class JS>
+__global__ void __launch_bounds__(128, 8)
+    k_shade_adj(Queue in, Queue out, AdjQueue ain, AdjQueue aout, WaveCounters *wcp, uint32_t wave, const float4 *hits,
+                const uint2 *hit_slot, float *g_alb, float *g_rough, const __grid_constant__ JS js) {
+  const WaveState &ws = wave_at(wcp, wave);
+  const uint32_t nf = ws.hit_count, n = nf + ws.hit_back, cap = wcp->cap;
+  unsigned *out_count = &wave_at(wcp, wave + 1).n_active;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) clear_wave(wcp, wave);
+  if ((t & ~31u) >= n) return;
+  bool enq = false;
+  float4 o4{}, d4{}, b4{}, rem4{}, l4{};
+  AdjTerms g{};
+  if (t < n) {
+    const uint32_t i = hit_index(t, nf, cap);
+    const uint2 hs = hit_slot[i];
+    o4 = in.o[hs.x], d4 = in.d[hs.x], b4 = in.beta[hs.x];
+    rem4 = ain.rem[hs.x], l4 = ain.dl[hs.x];
+    enq = shade_adj_path(o4, d4, b4, rem4, l4, hits[i], hs.y, wcp, js, g);
+  }
+  add_terms(g, g_alb, g_rough);
+  const unsigned slot = warp_append(enq, out_count);
   if (enq) {
-    out.o[slot] = no;
-    out.d[slot] = nd;
-    out.beta[slot] = nbeta;
-    aout.rem[slot] = nrem;
-    aout.dl[slot] = ndl;
+    out.o[slot] = o4;
+    out.d[slot] = d4;
+    out.beta[slot] = b4;
+    aout.rem[slot] = rem4;
+    aout.dl[slot] = l4;
   }
 }
 
-__global__ void k_wave_end(WaveCounters *wc) {
-  const uint32_t n_new = wave_new(*wc);
-  const uint32_t n = wc->n_active + n_new;
-  if (n) {
-    wc->waves++;
-    wc->traced += n;
+/* ---------------------------------------------------------------- finishing a draining wavefront
+ *
+ * Once every path has started and few are left, a wave costs the latency of its longest walk (70 us,
+ * 187 rays or 65,536 alike) whatever it holds, and each later bounce pays it again.  k_finish takes the
+ * queue instead and runs each path to its end in one thread: a warp waits for its own longest walk of
+ * each bounce, not the wave's, and the bounces need no launches.  The device functions are the waves'
+ * (same arithmetic per path, so the same films bit for bit).  A 256 x 256 frame of 65 k triangles, one
+ * sample, depth 4: five waves 440 us on the device, k_finish alone 235; 1283 x 721: 1.04 -> 0.87 ms. */
+constexpr int kFinishBlocks = 5; /* 96 registers; 4, 6 and 8 blocks per SM measured within 2 % */
+
+template <int WIDTH, class JS, bool ADJ>
+__global__ void __launch_bounds__(128, kFinishBlocks)
+    k_finish(Queue q, AdjQueue a, WaveCounters *wcp, uint32_t wave, float4 *L, float *g_alb, float *g_rough,
+             const __grid_constant__ JS js) {
+  const unsigned full = 0xffffffffu;
+  const uint32_t n = wave_rays(*wcp, wave_at(wcp, wave));
+  unsigned most = 0, sum = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; (i & ~31u) < n; i += gridDim.x * blockDim.x) {
+    bool alive = i < n;
+    float4 o4{}, d4{}, b4{}, rem4{}, l4{};
+    if (alive) {
+      o4 = q.o[i], d4 = q.d[i], b4 = q.beta[i];
+      if constexpr (ADJ) rem4 = a.rem[i], l4 = a.dl[i];
+    }
+    for (unsigned seg = 1; __any_sync(full, alive); seg++) {
+      float4 h{};
+      uint32_t inst = 0;
+      AdjTerms g{};
+      if (alive) {
+        const DevScene &sc = js.at(__float_as_uint(d4.w) >> 8).sc;
+        const TraceResult r = walk<WIDTH>(sc, V3{o4.x, o4.y, o4.z}, V3{d4.x, d4.y, d4.z});
+        h = make_float4(r.t, r.u, r.v, __int_as_float(r.prim));
+        inst = r.inst;
+        most = max(most, seg);
+        sum++;
+      }
+      __syncwarp();
+      if (alive) {
+        const DevScene &sc = js.at(__float_as_uint(d4.w) >> 8).sc;
+        if (__float_as_int(h.w) < 0) {
+          alive = false;
+          if constexpr (!ADJ) {
+            const V4 e = env_sample(sc, V3{d4.x, d4.y, d4.z});
+            finish_path(sc, L, __float_as_uint(o4.w),
+                        finite_or_zero(V3{b4.x, b4.y, b4.z} * V3{e.x, e.y, e.z},
+                                       (float)(__float_as_uint(d4.w) & 0xffu) + e.w, &wcp->nonfinite),
+                        &wcp->nonfinite);
+          }
+        } else if constexpr (ADJ) {
+          alive = shade_adj_path(o4, d4, b4, rem4, l4, h, inst, wcp, js, g);
+        } else {
+          alive = shade_path<JS, false>(o4, d4, b4, h, inst, wcp, L, js);
+        }
+      }
+      if constexpr (ADJ) {
+        __syncwarp();
+        add_terms(g, g_alb, g_rough);
+      }
+    }
   }
-  wc->next += n_new;
-  wc->n_active = wc->out_count;
-  wc->out_count = 0;
-  wc->hit_count = 0;
-  wc->hit_back = 0;
-  wc->trace_next = 0;
-  wc->shade_next = 0;
-  wc->done = (wc->n_active == 0 && wc->next == wc->total) ? 1u : 0u;
+  for (int off = 16; off > 0; off >>= 1) {
+    sum += __shfl_xor_sync(full, sum, off);
+    most = max(most, __shfl_xor_sync(full, most, off));
+  }
+  if ((threadIdx.x & 31u) == 0 && sum) {
+    atomicAdd(&wcp->traced, (unsigned long long)sum);
+    atomicMax(&wcp->finish_waves, most);
+  }
 }
 
 /* ---------------------------------------------------------------- persistent wavefront (trace_mode 3)
@@ -951,7 +921,8 @@ __global__ void __launch_bounds__(128, NB_PERSIST_MIN_BLOCKS) k_persist(Queue qa
   for (uint32_t w = 0;; w++) {
     const Queue &in = (w & 1u) ? qb : qa;
     const Queue &out = (w & 1u) ? qa : qb;
-    const uint32_t n_active = __ldcg(&wcp->n_active), next = __ldcg(&wcp->next);
+    WaveState &ws = wave_at(wcp, w);
+    const uint32_t n_active = __ldcg(&ws.n_active), next = __ldcg(&ws.next);
     const uint32_t total = __ldcg(&wcp->total), cap = __ldcg(&wcp->cap);
     if (__ldcg(&wcp->done)) return;
     const uint32_t n_new = min(cap - n_active, total - next), n = n_active + n_new;
@@ -959,35 +930,30 @@ __global__ void __launch_bounds__(128, NB_PERSIST_MIN_BLOCKS) k_persist(Queue qa
     if (!grid_barrier(sync, limit_ns)) return;
     const unsigned long long t0 = leader ? global_ns() : 0ull;
     for (;;) {
-      const uint32_t base = warp_take(&wcp->trace_next);
+      const uint32_t base = warp_take(&ws.trace_next);
       if (base >= n) break;
-      trace_warp<WIDTH, JS, false, false, true>(in, wcp, hits, hit_slot, L, js, base + lane, n);
+      trace_warp<WIDTH, JS, false, false, true>(in, wcp, ws, hits, hit_slot, L, js, base + lane, n);
     }
     if (!grid_barrier(sync, limit_ns)) return;
     const unsigned long long t1 = leader ? global_ns() : 0ull;
-    const uint32_t nh = __ldcg(&wcp->hit_count);
+    const uint32_t nh = __ldcg(&ws.hit_count);
+    unsigned *out_count = &wave_at(wcp, w + 1).n_active;
     for (;;) {
-      const uint32_t base = warp_take(&wcp->shade_next);
+      const uint32_t base = warp_take(&ws.shade_next);
       if (base >= nh) break;
-      shade_warp<JS, true>(in, out, wcp, hits, hit_slot, L, js, base + lane, nh);
+      shade_warp<JS, true>(in, out, wcp, out_count, hits, hit_slot, L, js, base + lane, base + lane < nh);
     }
     if (!grid_barrier(sync, limit_ns)) return;
-    if (leader) { /* k_wave_end's update */
+    if (leader) { /* the next entry's first path, the one after it cleared */
       sync->trace_ns += t1 - t0;
       sync->shade_ns += global_ns() - t1;
-      WaveCounters *wc = wcp;
       if (n) {
-        wc->waves++;
-        wc->traced += n;
+        wcp->waves++;
+        wcp->traced += n;
       }
-      wc->next = next + n_new;
-      wc->n_active = __ldcg(&wcp->out_count);
-      wc->out_count = 0;
-      wc->hit_count = 0;
-      wc->hit_back = 0;
-      wc->trace_next = 0;
-      wc->shade_next = 0;
-      wc->done = (wc->n_active == 0 && wc->next == total) ? 1u : 0u;
+      wave_at(wcp, w + 1).next = next + n_new;
+      clear_wave(wcp, w);
+      wcp->done = (__ldcg(out_count) == 0 && next + n_new == total) ? 1u : 0u;
       if (*cancel) atomicCAS(&sync->status, 0u, 2u);
       __threadfence();
     }
@@ -1086,17 +1052,15 @@ nova_b200_status ensure_film(nova_b200_ctx *c, int W, int H) {
 }
 
 nova_b200_status ensure_wave_buffers(nova_b200_ctx *c, uint32_t cap, size_t radiance) {
-  bool changed = false;
   if (c->queue_cap < cap) {
     cudaFree(c->d_queue);
     c->d_queue = nullptr;
     c->queue_cap = 0;
     c->queue_bytes = 0;
-    const size_t bytes = (size_t)cap * (16 * 7 + 8 + (NB_RAY_ORDER ? 4 : 0));
+    const size_t bytes = (size_t)cap * (16 * 7 + 8);
     NB_CUDA(c, cudaMalloc(&c->d_queue, bytes), "cudaMalloc(queue)");
     c->queue_cap = cap;
     c->queue_bytes = bytes;
-    changed = true;
   }
   if (c->radiance_cap < radiance) {
     cudaFree(c->d_radiance);
@@ -1104,20 +1068,13 @@ nova_b200_status ensure_wave_buffers(nova_b200_ctx *c, uint32_t cap, size_t radi
     c->radiance_cap = 0;
     NB_CUDA(c, cudaMalloc(&c->d_radiance, radiance * sizeof(float4)), "cudaMalloc(radiance)");
     c->radiance_cap = radiance;
-    changed = true;
   }
   if (!c->d_wave) {
     NB_CUDA(c, cudaMalloc(&c->d_wave, sizeof(WaveCounters)), "cudaMalloc(wave counters)");
     NB_CUDA(c, cudaMallocHost(&c->h_wave, 3 * sizeof(WaveCounters)), "cudaMallocHost(wave counters)");
-    for (int k = 0; k < 2 * 3 * kWavesPerGraph; k++) NB_CUDA(c, cudaEventCreate(&c->ev_wave[k]), "cudaEventCreate");
-    for (int k = 0; k < 2; k++)
-      NB_CUDA(c, cudaEventCreateWithFlags(&c->ev_done[k], cudaEventDisableTiming), "cudaEventCreate");
-    changed = true;
-  }
-  if (changed) {
-    for (cudaGraphExec_t &g : c->graph_exec)
-      if (g) cudaGraphExecDestroy(g), g = nullptr;
-    c->graph_key.clear();
+    for (cudaEvent_t &e : c->ev_wave) NB_CUDA(c, cudaEventCreate(&e), "cudaEventCreate");
+    for (cudaEvent_t &e : c->ev_done)
+      NB_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
   }
   return NOVA_B200_SUCCESS;
 }
@@ -1130,13 +1087,13 @@ struct LaunchShape {
                          2: one ray per thread, counting node visits and triangle tests,
                          3: the persistent wavefront (one cooperative launch per chunk) */
   uint32_t wait_limit_us; /* trace_mode 3: longest grid-barrier wait before the render fails */
+  uint32_t finish_rays;   /* rays left at which k_finish takes over (trace modes 1 and 2 stay with their kernel) */
 };
 
 struct WaveBuffers {
   Queue qa, qb;
   float4 *hits;
   uint2 *hit_slot; /* per hit: its ray's queue slot and the hit triangle's instance */
-  uint32_t *order; /* k_order_rays' slot order (NB_RAY_ORDER builds only) */
   WaveCounters *wc;
 };
 
@@ -1148,15 +1105,10 @@ WaveBuffers wave_buffers(nova_b200_ctx *c) {
   b.qb = Queue{base + 3 * (size_t)cap, base + 4 * (size_t)cap, base + 5 * (size_t)cap};
   b.hits = base + 6 * (size_t)cap;
   b.hit_slot = reinterpret_cast<uint2 *>(base + 7 * (size_t)cap);
-  b.order = NB_RAY_ORDER ? reinterpret_cast<uint32_t *>(b.hit_slot + cap) : nullptr;
   b.wc = static_cast<WaveCounters *>(c->d_wave);
   return b;
 }
 
-/* Enqueues one group of kWavesPerGraph waves for pipeline slot `slot` (queues alternating
- * A -> B -> A ...): an event record around each trace and shade kernel (`external` while capturing,
- * so they become graph event-record nodes), the read-back of the counters into the slot's pinned
- * copy and the slot's completion event. */
 /* Replay-loop arguments: the adjoint queues (A, B), the image adjoint and the gradients. */
 struct AdjArgs {
   AdjQueue qa, qb;
@@ -1164,108 +1116,18 @@ struct AdjArgs {
   float *g_alb, *g_rough;
 };
 
-template <class JS, int WIDTH, bool ADJ = false>
-void enqueue_waves(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, int slot, bool external,
-                   const AdjArgs *adj = nullptr) {
-  const WaveBuffers b = wave_buffers(c);
-  int dev_sms = 148, occ_r = 1;
-  cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_refill<JS>, 256, 0);
-  /* trace and shade: one ray per thread over the wave capacity, so the hardware block scheduler
-   * balances rays of very different cost; blocks past the live count exit at once */
-  const unsigned g_trace = (ls.cap + ls.trace_block - 1) / ls.trace_block;
-  const unsigned g_shade = (ls.cap + ls.shade_block - 1) / ls.shade_block;
-  const unsigned g_refill = (unsigned)(dev_sms * std::max(1, occ_r) * 2);
-  int occ_t = 1;
-  if (WIDTH == 2 && ls.trace_mode == 1)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_trace_dyn<JS>, 128, 0);
-  const unsigned g_dyn = (unsigned)std::min<uint64_t>((uint64_t)dev_sms * std::max(1, occ_t), (ls.cap + 127) / 128);
-  const unsigned flags = external ? cudaEventRecordExternal : cudaEventRecordDefault;
-  cudaEvent_t *ev = c->ev_wave + 3 * kWavesPerGraph * slot;
-  for (int w = 0; w < kWavesPerGraph; w++) {
-    const Queue &in = (w & 1) ? b.qb : b.qa;
-    const Queue &out = (w & 1) ? b.qa : b.qb;
-    if constexpr (ADJ) {
-      const AdjQueue &ain = (w & 1) ? adj->qb : adj->qa;
-      const AdjQueue &aout = (w & 1) ? adj->qa : adj->qb;
-      k_refill_adj<JS><<<g_refill, 256, 0, c->stream>>>(in, ain, b.wc, c->d_radiance, adj->d_image, js);
-      cudaEventRecordWithFlags(ev[3 * w + 0], c->stream, flags);
-      k_trace<WIDTH, JS, true><<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, b.hits, b.hit_slot, nullptr, js);
-      cudaEventRecordWithFlags(ev[3 * w + 1], c->stream, flags);
-      k_shade_adj<JS><<<g_shade, ls.shade_block, 0, c->stream>>>(in, out, ain, aout, b.wc, b.hits, b.hit_slot,
-                                                                 adj->g_alb, adj->g_rough, js);
-      cudaEventRecordWithFlags(ev[3 * w + 2], c->stream, flags);
-    } else {
-      k_refill<JS><<<g_refill, 256, 0, c->stream>>>(in, b.wc, c->d_radiance, js);
-      const bool ordered = NB_RAY_ORDER && !(WIDTH == 2 && ls.trace_mode == 1);
-#if NB_RAY_ORDER
-      if (ordered)
-        k_order_rays<NB_RAY_ORDER><<<(ls.cap + NB_RAY_ORDER - 1) / NB_RAY_ORDER, kOrderThreads, 0, c->stream>>>(
-            in, b.wc, b.order);
-#endif
-      const uint32_t *order = ordered ? b.order : nullptr;
-      cudaEventRecordWithFlags(ev[3 * w + 0], c->stream, flags);
-      if (WIDTH == 2 && ls.trace_mode == 1)
-        k_trace_dyn<JS><<<g_dyn, 128, 0, c->stream>>>(in, b.wc, b.hits, b.hit_slot, c->d_radiance, js);
-      else if (ls.trace_mode == 2)
-        k_trace<WIDTH, JS, false, true>
-            <<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, b.hits, b.hit_slot, c->d_radiance, js, order);
-      else
-        k_trace<WIDTH, JS>
-            <<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, b.hits, b.hit_slot, c->d_radiance, js, order);
-      cudaEventRecordWithFlags(ev[3 * w + 1], c->stream, flags);
-      k_shade<JS><<<g_shade, ls.shade_block, 0, c->stream>>>(in, out, b.wc, b.hits, b.hit_slot, c->d_radiance, js);
-      cudaEventRecordWithFlags(ev[3 * w + 2], c->stream, flags);
-    }
-    k_wave_end<<<1, 1, 0, c->stream>>>(b.wc);
-  }
-  cudaMemcpyAsync(static_cast<WaveCounters *>(c->h_wave) + slot, b.wc, sizeof(WaveCounters), cudaMemcpyDeviceToHost,
-                  c->stream);
-  cudaEventRecordWithFlags(c->ev_done[slot], c->stream, flags);
-}
+/* Rays up to which a wavefront with no path left to start goes to k_finish: about two rays for each of
+ * its 95,000 resident threads, above which a wave is bound by its rays and no longer by its longest walk.
+ * Fewer leave waves to their latency (75,000: a 256 x 256 x 16 adjoint step 1.53 ms against 1.44), more
+ * give up the waves' full warps (600,000: 1000 instances at 720p 5.6 ms against 4.5; 300,000: 4.7). */
+constexpr uint32_t kFinishRays = 150000;
 
-template <class JS>
-void enqueue_group(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, int width, int slot, bool external) {
-  if (width == 8)
-    enqueue_waves<JS, 8>(c, js, ls, slot, external);
-  else if (width == 1)
-    enqueue_waves<JS, 1>(c, js, ls, slot, external);
-  else
-    enqueue_waves<JS, 2>(c, js, ls, slot, external);
-}
-
-/* Batch chunks: each slot's group is captured into a CUDA graph for the chunk's job table (the
- * table is a kernel parameter); the graphs are kept while the same table and width come back. */
-nova_b200_status capture_graphs(nova_b200_ctx *c, const ManyJobs &js, const LaunchShape &ls, int width) {
-  const size_t key_bytes = sizeof(ManyJobs) + sizeof(LaunchShape) + sizeof(int);
-  std::vector<char> key(key_bytes);
-  std::memcpy(key.data(), &js, sizeof(ManyJobs));
-  std::memcpy(key.data() + sizeof(ManyJobs), &ls, sizeof(LaunchShape));
-  std::memcpy(key.data() + sizeof(ManyJobs) + sizeof(LaunchShape), &width, sizeof(int));
-  if (c->graph_exec[0] && c->graph_exec[1] && c->graph_key == key) return NOVA_B200_SUCCESS;
-  c->graph_key.clear();
-  for (int slot = 0; slot < 2; slot++) {
-    if (c->graph_exec[slot]) cudaGraphExecDestroy(c->graph_exec[slot]), c->graph_exec[slot] = nullptr;
-    cudaGraph_t graph = nullptr;
-    NB_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "capture");
-    enqueue_group(c, js, ls, width, slot, true);
-    const cudaError_t e_launch = cudaGetLastError();
-    const cudaError_t e_end = cudaStreamEndCapture(c->stream, &graph);
-    if (e_launch != cudaSuccess) {
-      if (graph) cudaGraphDestroy(graph);
-      return nbctx::cuda_fail(c, e_launch, "capture kernels");
-    }
-    if (e_end != cudaSuccess) return nbctx::cuda_fail(c, e_end, "cudaStreamEndCapture");
-    const cudaError_t e_inst = cudaGraphInstantiate(&c->graph_exec[slot], graph, 0);
-    cudaGraphDestroy(graph);
-    if (e_inst != cudaSuccess) {
-      c->graph_exec[slot] = nullptr;
-      return nbctx::cuda_fail(c, e_inst, "cudaGraphInstantiate");
-    }
-  }
-  c->graph_key = std::move(key);
-  return NOVA_B200_SUCCESS;
-}
+/* One wave to enqueue: its number, the most rays and new paths it can hold (its kernels read the exact
+ * counts on the device) and whether k_finish takes it over. */
+struct WavePlan {
+  uint32_t wave, rays, fresh;
+  bool finish;
+};
 
 /* Counters of wave loops. */
 struct LoopStats {
@@ -1287,39 +1149,127 @@ struct LoopStats {
   }
 };
 
-/* Runs the device-driven wave loop over `total` paths: uploads the counters, keeps two groups of
- * waves in flight (launch(slot) enqueues one), reads each finished group's counters and event
- * times, and stops once the device reports every path finished.  The group still in flight then
- * finds empty queues. */
+/* Enqueues one wave for pipeline slot wave & 1 (queues alternating A -> B -> A ...): an event record
+ * around the trace and the shading kernel (k_finish counts as the trace), the read-back of the counters
+ * into the slot's pinned copy and the slot's completion event. */
+template <class JS, int WIDTH, bool ADJ = false>
+cudaError_t enqueue_wave(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, const WavePlan &p, uint64_t &kernels,
+                         const AdjArgs *adj = nullptr) {
+  const WaveBuffers b = wave_buffers(c);
+  const int slot = (int)(p.wave & 1u);
+  const Queue &in = slot ? b.qb : b.qa, &out = slot ? b.qa : b.qb;
+  AdjQueue ain{}, aout{};
+  if constexpr (ADJ) ain = slot ? adj->qb : adj->qa, aout = slot ? adj->qa : adj->qb;
+  auto blocks = [](uint32_t n, uint32_t block) { return std::max(1u, (n + block - 1) / block); };
+  cudaEvent_t *ev = c->ev_wave + 3 * slot;
+  if (p.fresh) {
+    const unsigned g = blocks(p.fresh, 256);
+    if constexpr (ADJ)
+      k_refill_adj<JS><<<g, 256, 0, c->stream>>>(in, ain, b.wc, p.wave, c->d_radiance, adj->d_image, js);
+    else
+      k_refill<JS><<<g, 256, 0, c->stream>>>(in, b.wc, p.wave, c->d_radiance, js);
+    kernels++;
+  }
+  cudaEventRecord(ev[0], c->stream);
+  if (p.finish) {
+    k_finish<WIDTH, JS, ADJ><<<blocks(p.rays, 128), 128, 0, c->stream>>>(
+        in, ain, b.wc, p.wave, c->d_radiance, ADJ ? adj->g_alb : nullptr, ADJ ? adj->g_rough : nullptr, js);
+    kernels++;
+    cudaEventRecord(ev[1], c->stream);
+  } else {
+    const unsigned g_trace = blocks(p.rays, ls.trace_block);
+    const unsigned g_shade = blocks(p.rays, ls.shade_block);
+    if constexpr (ADJ) {
+      k_trace<WIDTH, JS, true>
+          <<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, p.wave, b.hits, b.hit_slot, nullptr, js);
+      cudaEventRecord(ev[1], c->stream);
+      k_shade_adj<JS><<<g_shade, ls.shade_block, 0, c->stream>>>(in, out, ain, aout, b.wc, p.wave, b.hits, b.hit_slot,
+                                                                 adj->g_alb, adj->g_rough, js);
+    } else {
+      if (WIDTH == 2 && ls.trace_mode == 1) {
+        int sms = 148, occ = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trace_dyn<JS>, 128, 0);
+        k_trace_dyn<JS><<<std::min(blocks(p.rays, 128), (unsigned)(sms * std::max(1, occ))), 128, 0, c->stream>>>(
+            in, b.wc, p.wave, b.hits, b.hit_slot, c->d_radiance, js);
+      } else if (ls.trace_mode == 2) {
+        k_trace<WIDTH, JS, false, true>
+            <<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, p.wave, b.hits, b.hit_slot, c->d_radiance, js);
+      } else {
+        k_trace<WIDTH, JS>
+            <<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, p.wave, b.hits, b.hit_slot, c->d_radiance, js);
+      }
+      cudaEventRecord(ev[1], c->stream);
+      k_shade<JS><<<g_shade, ls.shade_block, 0, c->stream>>>(in, out, b.wc, p.wave, b.hits, b.hit_slot, c->d_radiance,
+                                                             js);
+    }
+    kernels += 2;
+  }
+  cudaEventRecord(ev[2], c->stream);
+  cudaMemcpyAsync(static_cast<WaveCounters *>(c->h_wave) + slot, b.wc, sizeof(WaveCounters), cudaMemcpyDeviceToHost,
+                  c->stream);
+  cudaEventRecord(c->ev_done[slot], c->stream);
+  return cudaGetLastError();
+}
+
+/* The wave launcher of a job table: run_waves' `launch`. */
+template <bool ADJ = false, class JS>
+auto wave_launcher(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, int width, const AdjArgs *adj = nullptr) {
+  return [=, &js, &ls](const WavePlan &p, uint64_t &kernels) {
+    if (width == 8) return enqueue_wave<JS, 8, ADJ>(c, js, ls, p, kernels, adj);
+    if (width == 1) return enqueue_wave<JS, 1, ADJ>(c, js, ls, p, kernels, adj);
+    return enqueue_wave<JS, 2, ADJ>(c, js, ls, p, kernels, adj);
+  };
+}
+
+/* Runs the device-driven wave loop over `total` paths: uploads the counters, keeps two waves in flight
+ * (launch(plan, kernels) enqueues one), reads each finished wave's counters and event times, and stops
+ * once every path has ended.  A wave is enqueued while the one before it runs, so its plan holds upper
+ * bounds: the rays of that wave and the paths not yet started.  Once no path is left to start and at
+ * most `finish_rays` rays are, the plan is k_finish's and the last. */
 template <class Launch>
-nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, Launch &&launch, LoopStats &ls) {
+nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, uint32_t finish_rays, Launch &&launch,
+                           LoopStats &ls) {
   WaveCounters *hw = static_cast<WaveCounters *>(x->h_wave); /* [0], [1]: read-back slots, [2]: upload */
-  /* a previous loop's last (empty) group may still be running: it is stream-ordered before this
-   * upload, and the upload slot is only rewritten once the previous upload has completed */
   hw[2] = WaveCounters{};
   hw[2].total = total;
   hw[2].cap = cap;
   NB_CUDA(x, cudaMemcpyAsync(x->d_wave, hw + 2, sizeof(WaveCounters), cudaMemcpyHostToDevice, x->stream),
           "upload(wave counters)");
-  NB_CUDA(x, launch(0), "wave group");
-  NB_CUDA(x, launch(1), "wave group");
-  int slot = 0;
+  /* bounds on the next wave to enqueue: its waiting rays, and the paths started before it (exact) */
+  uint32_t waiting = 0, started = 0, enqueued = 0, finished = 0;
+  bool finish = false;
   for (;;) {
-    NB_CUDA(x, cudaEventSynchronize(x->ev_done[slot]), "waves");
-    const cudaEvent_t *ev = x->ev_wave + 3 * kWavesPerGraph * slot;
-    for (int w = 0; w < kWavesPerGraph; w++) {
-      float a = 0.f, b = 0.f;
-      cudaEventElapsedTime(&a, ev[3 * w], ev[3 * w + 1]);
-      cudaEventElapsedTime(&b, ev[3 * w + 1], ev[3 * w + 2]);
-      ls.t_trace += a;
-      ls.t_shade += b;
+    while (!finish && enqueued < finished + 2) {
+      WavePlan p{enqueued, 0, 0, false};
+      p.rays = (uint32_t)std::min<uint64_t>(cap, (uint64_t)waiting + (total - started));
+      if (p.rays == 0) break;
+      p.fresh = std::min(cap, total - started);
+      p.finish = finish = p.rays <= finish_rays && total - started <= cap - waiting;
+      NB_CUDA(x, launch(p, ls.kernels), "wave");
+      enqueued++;
+      /* at least cap - waiting of them start in this wave; how many exactly is read back */
+      started += std::min(cap - waiting, total - started);
+      waiting = p.rays;
     }
-    ls.kernels += 4 * kWavesPerGraph;
+    const int slot = (int)(finished & 1u);
+    NB_CUDA(x, cudaEventSynchronize(x->ev_done[slot]), "waves");
+    const cudaEvent_t *ev = x->ev_wave + 3 * slot;
+    float a = 0.f, b = 0.f;
+    cudaEventElapsedTime(&a, ev[0], ev[1]);
+    cudaEventElapsedTime(&b, ev[1], ev[2]);
+    ls.t_trace += a;
+    ls.t_shade += b;
     const WaveCounters r = hw[slot];
-    if (r.bad_index) { /* the device status word: stop after this group, as the reference aborts a tile
+    finished++;
+    auto drain = [&] { /* the wave still in flight; its counters */
+      if (enqueued == finished) return cudaSuccess;
+      return cudaEventSynchronize(x->ev_done[finished & 1u]);
+    };
+    if (r.bad_index) { /* the device status word: stop after this wave, as the reference aborts a tile
                         * once its exception manager holds an error (integrator/Integrator.h:74-78) */
-      NB_CUDA(x, cudaEventSynchronize(x->ev_done[slot ^ 1]), "waves");
-      const WaveCounters last = hw[slot ^ 1];
+      NB_CUDA(x, drain(), "waves");
+      const WaveCounters last = enqueued == finished ? r : hw[slot ^ 1];
       ls.bad_index += std::max(r.bad_index, last.bad_index);
       ls.nonfinite += std::max(r.nonfinite, last.nonfinite);
       char msg[160];
@@ -1327,23 +1277,30 @@ nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, Launc
                     (unsigned)std::max(r.bad_index, last.bad_index));
       return nbctx::fail(x, NOVA_B200_RENDERER_EXCEPTION, "%s", msg);
     }
-    if (r.done) {
-      ls.waves += r.waves;
+    const WaveState &next = r.w[finished % kWaveRing];
+    const bool done = finish ? finished == enqueued : next.n_active == 0 && next.next == total;
+    if (done) {
+      ls.waves += r.waves + r.finish_waves;
       ls.traced += r.traced;
       ls.nonfinite += r.nonfinite;
       ls.node_visits += r.node_visits;
       ls.tri_tests += r.tri_tests;
-      break;
+      return NOVA_B200_SUCCESS;
     }
-    if (x->cancel.load()) { /* nova_b200_cancel: let the group in flight finish, enqueue nothing more */
-      NB_CUDA(x, cudaEventSynchronize(x->ev_done[slot ^ 1]), "waves");
+    if (x->cancel.load()) { /* nova_b200_cancel: let the wave in flight finish, enqueue nothing more */
+      NB_CUDA(x, drain(), "waves");
       return nbctx::fail(x, NOVA_B200_RENDERER_EXCEPTION, "render cancelled%s");
     }
-    NB_CUDA(x, launch(slot), "wave group");
-    slot ^= 1;
+    /* the counts before wave `finished` are known now; a wave already enqueued after it starts what its
+     * queue has room for and leaves at most its rays */
+    waiting = next.n_active;
+    started = next.next;
+    for (uint32_t w = finished; w < enqueued; w++) {
+      const uint32_t fresh = std::min(cap - waiting, total - started);
+      started += fresh;
+      waiting += fresh;
+    }
   }
-  ls.kernels += 4 * kWavesPerGraph; /* the empty group */
-  return NOVA_B200_SUCCESS;
 }
 
 /* The persistent wavefront over `total` paths: counters and barrier reset, one cooperative launch of
@@ -1493,7 +1450,7 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
   const uint32_t qc = tu.queue_capacity ? tu.queue_capacity : kQueueCapDefault;
   const uint32_t cap = (uint32_t)std::min<uint64_t>(qc, std::max<uint64_t>(radiance, 1024));
   const LaunchShape ls{cap, tu.trace_block ? tu.trace_block : 128u, tu.shade_block ? tu.shade_block : 128u,
-                       tu.trace_mode, tu.wait_limit_us ? tu.wait_limit_us : 1000000u};
+                       tu.trace_mode, tu.wait_limit_us ? tu.wait_limit_us : 1000000u, tu.trace_mode ? 0u : kFinishRays};
   nova_b200_status st = ensure_wave_buffers(x, cap, radiance);
   if (st != NOVA_B200_SUCCESS) return st;
   x->primal_valid = false; /* this render overwrites the radiance buffer */
@@ -1622,18 +1579,12 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
       many.n = (uint32_t)chunk.size();
       std::copy(hj.begin(), hj.begin() + chunk.size(), many.j);
     }
-    if (ls.trace_mode == 3) { /* the persistent wavefront: one launch runs every wave of the chunk */
+    if (ls.trace_mode == 3) /* the persistent wavefront: one launch runs every wave of the chunk */
       st = single ? run_persistent_w(x, one, ls, width, pb, cap, loop) : run_persistent_w(x, many, ls, width, pb, cap, loop);
-      if (st != NOVA_B200_SUCCESS) return st;
-    } else {
-      if (!single && (st = capture_graphs(x, many, ls, width)) != NOVA_B200_SUCCESS) return st;
-      auto launch = [&](int slot) {
-        if (!single) return cudaGraphLaunch(x->graph_exec[slot], x->stream);
-        enqueue_group(x, one, ls, width, slot, false);
-        return cudaGetLastError();
-      };
-      if ((st = run_waves(x, pb, cap, launch, loop)) != NOVA_B200_SUCCESS) return st;
-    }
+    else
+      st = single ? run_waves(x, pb, cap, ls.finish_rays, wave_launcher(x, one, ls, width), loop)
+                  : run_waves(x, pb, cap, ls.finish_rays, wave_launcher(x, many, ls, width), loop);
+    if (st != NOVA_B200_SUCCESS) return st;
     sum.paths += pb;
     for (size_t k = 0; k < chunk.size(); k++) {
       const Piece &P = chunk[k];
@@ -1818,7 +1769,8 @@ nova_b200_status nb_backward(nova_b200_ctx *c, const nova_b200_frame *f, const f
   const uint32_t qc = tu.queue_capacity ? tu.queue_capacity : kQueueCapDefault;
   const uint32_t cap = (uint32_t)std::min<uint64_t>(qc, std::max<uint64_t>(radiance, 1024));
   const LaunchShape ls{cap, tu.trace_block ? tu.trace_block : 128u, tu.shade_block ? tu.shade_block : 128u,
-                       tu.trace_mode == 3 ? 0u : tu.trace_mode, 0u}; /* the replay keeps the per-wave kernels */
+                       tu.trace_mode == 3 ? 0u : tu.trace_mode, 0u, /* the replay keeps the per-wave kernels */
+                       tu.trace_mode == 1 || tu.trace_mode == 2 ? 0u : kFinishRays};
   if ((st = ensure_wave_buffers(c, cap, radiance)) != NOVA_B200_SUCCESS) return st;
   if (c->adj_cap < c->queue_cap) {
     cudaFree(c->d_adj);
@@ -1864,22 +1816,13 @@ nova_b200_status nb_backward(nova_b200_ctx *c, const nova_b200_frame *f, const f
     J.path_begin = 0;
     J.n_paths = NP * take;
     /* primal: each path's radiance into the radiance buffer */
-    auto fwd = [&](int slot) {
-      enqueue_group(c, one, ls, width, slot, false);
-      return cudaGetLastError();
-    };
-    if (!reuse && (st = run_waves(c, J.n_paths, cap, fwd, primal)) != NOVA_B200_SUCCESS) return st;
+    if (!reuse &&
+        (st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher(c, one, ls, width), primal)) != NOVA_B200_SUCCESS)
+      return st;
     /* replay with the adjoint */
-    auto bwd = [&](int slot) {
-      if (width == 8)
-        enqueue_waves<OneJob, 8, true>(c, one, ls, slot, false, &adj);
-      else if (width == 1)
-        enqueue_waves<OneJob, 1, true>(c, one, ls, slot, false, &adj);
-      else
-        enqueue_waves<OneJob, 2, true>(c, one, ls, slot, false, &adj);
-      return cudaGetLastError();
-    };
-    if ((st = run_waves(c, J.n_paths, cap, bwd, replay)) != NOVA_B200_SUCCESS) return st;
+    if ((st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher<true>(c, one, ls, width, &adj), replay)) !=
+        NOVA_B200_SUCCESS)
+      return st;
     sum.paths += J.n_paths;
   }
   NB_CUDA(c, cudaEventRecord(c->ev_end, c->stream), "event");

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128) k_path_noalloc(DevScene sc, Params rp, fl
   float4 lacc = make_float4(0.f, 0.f, 0.f, 0.f);
   float4 result = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int bounce = 0;; bounce++) {
-    const TraceResult h = trace_closest(sc, ro, rd);
+    const TraceResult h = walk_any(sc, ro, rd);
     if (h.prim < 0) {
       const V4 e = env_sample(sc, rd);
       result = finite_or_zero(beta * V3{e.x, e.y, e.z}, (float)bounce + e.w);

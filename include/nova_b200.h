@@ -141,14 +141,14 @@ typedef struct {
   uint64_t traced;     /* closest-hit queries issued on the device */
   uint64_t waves;      /* wavefront iterations */
   double device_ms;    /* device time of the render (CUDA events) */
-  double trace_ms;     /* device time inside the closest-hit kernel */
+  double trace_ms;     /* device time inside the closest-hit kernel, and the kernel that finishes the last paths */
   double shade_ms;     /* device time inside the shading kernel */
   uint64_t kernels;    /* kernels launched */
   /* The device status word of the call.  nonfinite: path radiance values that came out NaN or
    * infinite and were written as 0, as the reference's DENAN does (integrator/Integrator.cpp:92); the
    * render succeeds.  bad_index: hits whose primitive, instance or material id lies outside the
    * scene's tables (not reachable through validated uploads; it guards against corrupted device
-   * memory): the path ends black, the loop stops after the current wave group and the call returns
+   * memory): the path ends black, the loop stops after the current wave and the call returns
    * RENDERER_EXCEPTION, which the engine facade reports as exception::GENERAL_GPU_ERROR. */
   uint64_t nonfinite;
   uint64_t bad_index;
@@ -418,8 +418,8 @@ nova_b200_status nova_b200_last_call_ms(nova_b200_ctx *ctx, float *device_ms);
 
 /* Stops the render, render_batch or backward call running on this context (for a batch: on its
  * first context) from another thread: NvEngineInstance::stopRender's is_rendering flag
- * (api/engine.cpp:577-586).  The wave loop checks it after every group of four waves and between
- * chunks; the call then waits for the group still in flight and returns RENDERER_EXCEPTION
+ * (api/engine.cpp:577-586).  The wave loop checks it after every wave and between
+ * chunks; the call then waits for the wave still in flight and returns RENDERER_EXCEPTION
  * ("render cancelled") without writing the film (a batch spanning several chunks has already
  * written the films of frames that finished in an earlier chunk, when they are device or pinned
  * host buffers).  The accumulation film keeps the chunks finished before the stop, so the next
