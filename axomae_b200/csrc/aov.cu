@@ -38,9 +38,11 @@ constexpr int kAovBlocks = KIND == NOVA_B200_AOV_DEPTH ? 10 : KIND == NOVA_B200_
  * registers, 5 resident blocks for a walk that waits on its node loads. */
 template <int WIDTH, int KIND>
 __global__ void __launch_bounds__(128, kAovBlocks<KIND>) k_aov(DevScene sc, const AovParams p, float4 *out) {
-  const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= (uint32_t)p.W * (uint32_t)p.H) return;
-  const int y = (int)(pix / (uint32_t)p.W), x = (int)(pix - (uint32_t)y * (uint32_t)p.W);
+  /* a warp takes a tile of 8 x 4 pixels and a block 16 x 8: neighbouring rays walk alike */
+  const uint32_t tiles_x = ((uint32_t)p.W + 15u) / 16u, w = threadIdx.x >> 5;
+  const int x = (int)(blockIdx.x % tiles_x * 16u + (w & 1u) * 8u + (threadIdx.x & 7u));
+  const int y = (int)(blockIdx.x / tiles_x * 8u + (w >> 1) * 4u + (threadIdx.x >> 3 & 3u));
+  if (x >= p.W || y >= p.H) return;
   const int ys = p.H - y; /* screen row, as the path integrator */
   const float nx = (float)(2 * x - p.W) / (float)p.W;
   const float ny = (float)(p.H - 2 * ys) / (float)p.H;
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(128, kAovBlocks<KIND>) k_aov(DevScene sc, cons
 
 template <int WIDTH>
 void launch_aov(nova_b200_ctx *c, int32_t kind, const AovParams &p, float4 *out) {
-  const unsigned grid = (unsigned)(((size_t)p.W * p.H + 127) / 128);
+  const unsigned grid = (unsigned)((((size_t)p.W + 15) / 16) * (((size_t)p.H + 7) / 8));
   if (kind == NOVA_B200_AOV_DEPTH)
     k_aov<WIDTH, NOVA_B200_AOV_DEPTH><<<grid, 128, 0, c->stream>>>(c->scene, p, out);
   else if (kind == NOVA_B200_AOV_NORMAL)

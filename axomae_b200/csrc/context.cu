@@ -1018,10 +1018,9 @@ nova_b200_status nova_b200_build_bvh(nova_b200_ctx *c, const nova_b200_bvh_optio
   const uint32_t *d_valid = c->d_valid;
   uint32_t *d_order = nullptr;
   float4 *d_lo = nullptr, *d_hi = nullptr;
-  const size_t max_nodes = std::max<size_t>(2 * (size_t)n, 2);
+  const size_t max_nodes = (size_t)n + 1;
   NB_CUDA(c, cudaMallocAsync(&c->d_nodes, sizeof(float4) * 4 * max_nodes, c->stream), "cudaMalloc(nodes)");
   NB_CUDA(c, cudaMallocAsync(&c->d_tris, sizeof(float4) * (nb::kTriStride * (size_t)n + nb::kTriPad), c->stream), "cudaMalloc(tris)");
-  NB_CUDA(c, cudaMemsetAsync(c->d_nodes, 0, sizeof(float4) * 4 * max_nodes, c->stream), "memset(nodes)");
   NB_CUDA(c, cudaMallocAsync(&d_order, sizeof(uint32_t) * n, c->stream), "cudaMalloc(order)");
   NB_CUDA(c, cudaMallocAsync(&d_lo, sizeof(float4) * n, c->stream), "cudaMalloc(lo)");
   NB_CUDA(c, cudaMallocAsync(&d_hi, sizeof(float4) * n, c->stream), "cudaMalloc(hi)");
