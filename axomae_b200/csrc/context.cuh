@@ -49,6 +49,7 @@ struct nova_b200_ctx {
   float4 *d_film_acc = nullptr; /* running sum, row-major */
   int film_w = 0, film_h = 0;
   uint64_t film_samples = 0;
+  bool film_clear = false;      /* the running sum counts as zero, whatever the buffer holds */
   void *d_queue = nullptr;
   size_t queue_bytes = 0;
   uint32_t queue_cap = 0;

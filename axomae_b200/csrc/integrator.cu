@@ -961,11 +961,13 @@ __global__ void __launch_bounds__(128, NB_PERSIST_MIN_BLOCKS) k_persist(Queue qa
   }
 }
 
-__global__ void k_resolve(const float4 *L, uint32_t NP, uint32_t count, float4 *acc, float denom, float *out, int W,
-                          int H, int vinv) {
+/* Adds the chunk's samples of each pixel to its running sum (from zero when `clear`) and writes the mean;
+ * nothing once the device status word holds a bad index (the call fails). */
+__global__ void k_resolve(const float4 *L, uint32_t NP, uint32_t count, float4 *acc, bool clear, float denom, float *out,
+                          int W, int H, int vinv, const WaveCounters *wcp) {
   const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= NP) return;
-  float4 a = acc[pix];
+  if (pix >= NP || wcp->bad_index) return;
+  float4 a = clear ? make_float4(0.f, 0.f, 0.f, 0.f) : acc[pix];
   for (uint32_t s = 0; s < count; s++) {
     const float4 l = L[(size_t)s * NP + pix];
     a.x += l.x, a.y += l.y, a.z += l.z, a.w += l.w;
@@ -1037,7 +1039,7 @@ nova_b200_status ensure_film(nova_b200_ctx *c, int W, int H) {
     cudaFree(c->d_film_acc);
     c->d_film_acc = nullptr;
     NB_CUDA(c, cudaMalloc(&c->d_film_acc, npx * sizeof(float4)), "cudaMalloc(film)");
-    NB_CUDA(c, cudaMemsetAsync(c->d_film_acc, 0, npx * sizeof(float4), c->stream), "memset(film)");
+    c->film_clear = true;
     c->film_w = W;
     c->film_h = H;
     c->film_samples = 0;
@@ -1226,10 +1228,11 @@ auto wave_launcher(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, int wi
  * (launch(plan, kernels) enqueues one), reads each finished wave's counters and event times, and stops
  * once every path has ended.  A wave is enqueued while the one before it runs, so its plan holds upper
  * bounds: the rays of that wave and the paths not yet started.  Once no path is left to start and at
- * most `finish_rays` rays are, the plan is k_finish's and the last. */
-template <class Launch>
+ * most `finish_rays` rays are, the plan is k_finish's and the last.  after_last() enqueues what follows the
+ * last wave; behind k_finish the GPU goes on with it while the host still waits for the counters. */
+template <class Launch, class Last>
 nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, uint32_t finish_rays, Launch &&launch,
-                           LoopStats &ls) {
+                           Last &&after_last, LoopStats &ls) {
   WaveCounters *hw = static_cast<WaveCounters *>(x->h_wave); /* [0], [1]: read-back slots, [2]: upload */
   hw[2] = WaveCounters{};
   hw[2].total = total;
@@ -1248,6 +1251,7 @@ nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, uint3
       p.finish = finish = p.rays <= finish_rays && total - started <= cap - waiting;
       NB_CUDA(x, launch(p, ls.kernels), "wave");
       enqueued++;
+      if (finish) after_last();
       /* at least cap - waiting of them start in this wave; how many exactly is read back */
       started += std::min(cap - waiting, total - started);
       waiting = p.rays;
@@ -1285,9 +1289,11 @@ nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, uint3
       ls.nonfinite += r.nonfinite;
       ls.node_visits += r.node_visits;
       ls.tri_tests += r.tri_tests;
+      if (!finish) after_last();
       return NOVA_B200_SUCCESS;
     }
-    if (x->cancel.load()) { /* nova_b200_cancel: let the wave in flight finish, enqueue nothing more */
+    if (!finish && x->cancel.load()) { /* nova_b200_cancel: let the wave in flight finish, enqueue nothing
+                                        * more (a render whose last wave is enqueued completes) */
       NB_CUDA(x, drain(), "waves");
       return nbctx::fail(x, NOVA_B200_RENDERER_EXCEPTION, "render cancelled%s");
     }
@@ -1458,9 +1464,7 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
     nova_b200_ctx *c = ctxs[j];
     if ((st = ensure_film(c, frames[j]->width, frames[j]->height)) != NOVA_B200_SUCCESS) return st;
     if (frames[j]->reset) {
-      NB_CUDA(x, cudaMemsetAsync(c->d_film_acc, 0, (size_t)frames[j]->width * frames[j]->height * sizeof(float4),
-                                 x->stream),
-              "memset(film)");
+      c->film_clear = true; /* the next resolve starts from zero */
       c->film_samples = 0;
     }
   }
@@ -1497,11 +1501,11 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
   const size_t nc = chunks.size();
   std::vector<size_t> last_chunk(nj, 0);
   std::vector<char> early(nj, 0);
+  for (size_t ci = 0; ci < nc; ci++)
+    for (const Piece &P : chunks[ci])
+      for (size_t j = 0; j < nj; j++)
+        if (ctxs[j] == P.ctx) last_chunk[j] = ci;
   if (nc > 1) {
-    for (size_t ci = 0; ci < nc; ci++)
-      for (const Piece &P : chunks[ci])
-        for (size_t j = 0; j < nj; j++)
-          if (ctxs[j] == P.ctx) last_chunk[j] = ci;
     for (size_t j = 0; j < nj; j++) {
       bool pinned = false;
       if (films_host && films_host[j]) {
@@ -1525,14 +1529,20 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
       if (s) cudaStreamSynchronize(s);
     }
   } copies_done{nc > 1 ? x->copy_stream : nullptr};
+  /* where a frame's last resolve writes its film: the caller's device film itself when it is aligned, which
+   * saves a copy of it; earlier chunks of the frame write the context's, so that a render that fails
+   * leaves the caller's alone */
+  auto film_target = [&](size_t j) {
+    float *f = films_device ? films_device[j] : nullptr;
+    return f && !(reinterpret_cast<uintptr_t>(f) & 15u) ? f : ctxs[j]->d_film_out;
+  };
   auto copy_film = [&](size_t j, cudaStream_t stream) -> nova_b200_status {
     const size_t bytes = (size_t)frames[j]->width * frames[j]->height * 4 * sizeof(float);
-    if (films_device && films_device[j])
-      NB_CUDA(x, cudaMemcpyAsync(films_device[j], ctxs[j]->d_film_out, bytes, cudaMemcpyDeviceToDevice, stream),
-              "copy film");
+    const float *film = film_target(j);
+    if (films_device && films_device[j] && films_device[j] != film)
+      NB_CUDA(x, cudaMemcpyAsync(films_device[j], film, bytes, cudaMemcpyDeviceToDevice, stream), "copy film");
     if (films_host && films_host[j])
-      NB_CUDA(x, cudaMemcpyAsync(films_host[j], ctxs[j]->d_film_out, bytes, cudaMemcpyDeviceToHost, stream),
-              "copy film");
+      NB_CUDA(x, cudaMemcpyAsync(films_host[j], film, bytes, cudaMemcpyDeviceToHost, stream), "copy film");
     return NOVA_B200_SUCCESS;
   };
   nova_b200_render_stats sum{};
@@ -1579,23 +1589,36 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
       many.n = (uint32_t)chunk.size();
       std::copy(hj.begin(), hj.begin() + chunk.size(), many.j);
     }
-    if (ls.trace_mode == 3) /* the persistent wavefront: one launch runs every wave of the chunk */
+    /* the chunk's samples into its films, enqueued behind its last wave */
+    auto resolve = [&] {
+      for (size_t k = 0; k < chunk.size(); k++) {
+        const Piece &P = chunk[k];
+        nova_b200_ctx *c = P.ctx;
+        const size_t j = (size_t)(std::find(ctxs.begin(), ctxs.end(), c) - ctxs.begin());
+        c->film_samples += P.count;
+        const uint32_t NP = hj[k].rp.NP;
+        k_resolve<<<(NP + 255) / 256, 256, 0, x->stream>>>(
+            x->d_radiance + hj[k].path_begin, NP, P.count, c->d_film_acc, c->film_clear, (float)c->film_samples,
+            last_chunk[j] == ci ? film_target(j) : c->d_film_out, P.f->width, P.f->height, P.f->vertical_invert,
+            static_cast<const WaveCounters *>(x->d_wave));
+        c->film_clear = false;
+        sum.kernels++;
+      }
+    };
+    if (ls.trace_mode == 3) { /* the persistent wavefront: one launch runs every wave of the chunk */
       st = single ? run_persistent_w(x, one, ls, width, pb, cap, loop) : run_persistent_w(x, many, ls, width, pb, cap, loop);
-    else
-      st = single ? run_waves(x, pb, cap, ls.finish_rays, wave_launcher(x, one, ls, width), loop)
-                  : run_waves(x, pb, cap, ls.finish_rays, wave_launcher(x, many, ls, width), loop);
+      if (st == NOVA_B200_SUCCESS) resolve();
+    } else {
+      std::vector<std::pair<uint64_t, bool>> film_state; /* for a failure found after the resolves are enqueued */
+      for (const Piece &P : chunk) film_state.emplace_back(P.ctx->film_samples, P.ctx->film_clear);
+      st = single ? run_waves(x, pb, cap, ls.finish_rays, wave_launcher(x, one, ls, width), resolve, loop)
+                  : run_waves(x, pb, cap, ls.finish_rays, wave_launcher(x, many, ls, width), resolve, loop);
+      if (st != NOVA_B200_SUCCESS)
+        for (size_t k = 0; k < chunk.size(); k++)
+          chunk[k].ctx->film_samples = film_state[k].first, chunk[k].ctx->film_clear = film_state[k].second;
+    }
     if (st != NOVA_B200_SUCCESS) return st;
     sum.paths += pb;
-    for (size_t k = 0; k < chunk.size(); k++) {
-      const Piece &P = chunk[k];
-      nova_b200_ctx *c = P.ctx;
-      c->film_samples += P.count;
-      const uint32_t NP = hj[k].rp.NP;
-      k_resolve<<<(NP + 255) / 256, 256, 0, x->stream>>>(x->d_radiance + hj[k].path_begin, NP, P.count, c->d_film_acc,
-                                                         (float)c->film_samples, c->d_film_out, P.f->width,
-                                                         P.f->height, P.f->vertical_invert);
-      sum.kernels++;
-    }
     bool any = false;
     for (size_t j = 0; j < nj; j++) any = any || (early[j] && last_chunk[j] == ci);
     if (any) {
@@ -1817,10 +1840,10 @@ nova_b200_status nb_backward(nova_b200_ctx *c, const nova_b200_frame *f, const f
     J.n_paths = NP * take;
     /* primal: each path's radiance into the radiance buffer */
     if (!reuse &&
-        (st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher(c, one, ls, width), primal)) != NOVA_B200_SUCCESS)
+        (st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher(c, one, ls, width), [] {}, primal)) != NOVA_B200_SUCCESS)
       return st;
     /* replay with the adjoint */
-    if ((st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher<true>(c, one, ls, width, &adj), replay)) !=
+    if ((st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher<true>(c, one, ls, width, &adj), [] {}, replay)) !=
         NOVA_B200_SUCCESS)
       return st;
     sum.paths += J.n_paths;
