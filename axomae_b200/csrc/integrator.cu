@@ -248,11 +248,24 @@ __device__ __forceinline__ void refill_one(const Queue &q, uint32_t next, uint32
   if (js.at(c.job).sc.has_emissive) L[c.rslot] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+/* The wave's counters; wave 0's refill starts them (no copy from the host before it), so its blocks take
+ * them as zero. */
+__device__ __forceinline__ WaveState first_state(WaveCounters *wcp, uint32_t wave, uint32_t total, uint32_t cap) {
+  if (wave != 0) return wave_at(wcp, wave);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    WaveCounters wc{};
+    wc.total = total;
+    wc.cap = cap;
+    *wcp = wc;
+  }
+  return WaveState{};
+}
+
 template <class JS>
-__global__ void __launch_bounds__(256) k_refill(Queue q, WaveCounters *wcp, uint32_t wave, float4 *L,
-                                                const __grid_constant__ JS js) {
-  const WaveState ws = wave_at(wcp, wave);
-  const uint32_t n_new = wave_new(*wcp, ws);
+__global__ void __launch_bounds__(256) k_refill(Queue q, WaveCounters *wcp, uint32_t wave, uint32_t total,
+                                                uint32_t cap, float4 *L, const __grid_constant__ JS js) {
+  const WaveState ws = first_state(wcp, wave, total, cap);
+  const uint32_t n_new = min(cap - ws.n_active, total - ws.next);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += gridDim.x * blockDim.x)
     refill_one(q, ws.next, ws.n_active, L, js, i);
 }
@@ -649,10 +662,10 @@ __device__ __forceinline__ void warp_add_by_key(bool active, uint32_t key, const
 
 template <class JS>
 __global__ void __launch_bounds__(256) k_refill_adj(Queue q, AdjQueue a, WaveCounters *wcp, uint32_t wave,
-                                                    const float4 *L, const float4 *d_image,
-                                                    const __grid_constant__ JS js) {
-  const WaveState ws = wave_at(wcp, wave);
-  const uint32_t n_new = wave_new(*wcp, ws);
+                                                    uint32_t total, uint32_t cap, const float4 *L,
+                                                    const float4 *d_image, const __grid_constant__ JS js) {
+  const WaveState ws = first_state(wcp, wave, total, cap);
+  const uint32_t n_new = min(cap - ws.n_active, total - ws.next);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += gridDim.x * blockDim.x) {
     const CameraPath c = camera_path(js, ws.next + i);
     const RenderParams &rp = js.at(c.job).rp;
@@ -783,13 +796,16 @@ constexpr int kFinishBlocks = 5; /* 96 registers; 4, 6 and 8 blocks per SM measu
 
 template <int WIDTH, class JS, bool ADJ>
 __global__ void __launch_bounds__(128, kFinishBlocks)
-    k_finish(Queue q, AdjQueue a, WaveCounters *wcp, uint32_t wave, float4 *L, float *g_alb, float *g_rough,
-             const __grid_constant__ JS js) {
+    k_finish(Queue q, AdjQueue a, WaveCounters *wcp, uint32_t wave, uint32_t lanes, float4 *L, float *g_alb,
+             float *g_rough, const __grid_constant__ JS js) {
   const unsigned full = 0xffffffffu;
   const uint32_t n = wave_rays(*wcp, wave_at(wcp, wave));
   unsigned most = 0, sum = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; (i & ~31u) < n; i += gridDim.x * blockDim.x) {
-    bool alive = i < n;
+  const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * blockDim.x + threadIdx.x) / 32u * lanes;
+  if (first >= n) return;
+  {
+    const uint32_t i = first + lane;
+    bool alive = lane < lanes && i < n;
     float4 o4{}, d4{}, b4{}, rem4{}, l4{};
     if (alive) {
       o4 = q.o[i], d4 = q.d[i], b4 = q.beta[i];
@@ -964,8 +980,9 @@ __global__ void __launch_bounds__(128, NB_PERSIST_MIN_BLOCKS) k_persist(Queue qa
 /* Adds the chunk's samples of each pixel to its running sum (from zero when `clear`) and writes the mean;
  * nothing once the device status word holds a bad index (the call fails). */
 __global__ void k_resolve(const float4 *L, uint32_t NP, uint32_t count, float4 *acc, bool clear, float denom, float *out,
-                          int W, int H, int vinv, const WaveCounters *wcp) {
+                          int W, int H, int vinv, const WaveCounters *wcp, WaveCounters *back) {
   const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pix == 0 && back) *back = *wcp; /* pinned host memory: read after the stream has been waited for */
   if (pix >= NP || wcp->bad_index) return;
   float4 a = clear ? make_float4(0.f, 0.f, 0.f, 0.f) : acc[pix];
   for (uint32_t s = 0; s < count; s++) {
@@ -1124,10 +1141,22 @@ struct AdjArgs {
  * give up the waves' full warps (600,000: 1000 instances at 720p 5.6 ms against 4.5; 300,000: 4.7). */
 constexpr uint32_t kFinishRays = 150000;
 
+/* Paths per warp of k_finish: the fewest, down to 2, that make at most 2,048 warps of paths already on
+ * their way, or 4,096 of camera rays, half of which end at once (2,960 warps are resident).  A warp takes
+ * as long as the union of its lanes' walks, so few paths are spread thin: 16,384 camera paths of depth 4
+ * take 146 us with 8 a warp and 185 with 32, 1,024 take 84 with 2 and 157 with 32; 65,536 take 173 with
+ * 16, 191 with 32 and 200 with 8, but the late waves of a 1283 x 721 frame lose 50 us with 16. */
+uint32_t finish_lanes(uint32_t rays, uint32_t wave) {
+  const uint32_t warps = wave == 0 ? 4096 : 2048;
+  uint32_t lanes = 32;
+  while (lanes > 2 && rays / (lanes / 2) <= warps) lanes /= 2;
+  return lanes;
+}
+
 /* One wave to enqueue: its number, the most rays and new paths it can hold (its kernels read the exact
  * counts on the device) and whether k_finish takes it over. */
 struct WavePlan {
-  uint32_t wave, rays, fresh;
+  uint32_t wave, rays, fresh, total, cap;
   bool finish;
 };
 
@@ -1167,17 +1196,19 @@ cudaError_t enqueue_wave(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, 
   if (p.fresh) {
     const unsigned g = blocks(p.fresh, 256);
     if constexpr (ADJ)
-      k_refill_adj<JS><<<g, 256, 0, c->stream>>>(in, ain, b.wc, p.wave, c->d_radiance, adj->d_image, js);
+      k_refill_adj<JS><<<g, 256, 0, c->stream>>>(in, ain, b.wc, p.wave, p.total, p.cap, c->d_radiance, adj->d_image, js);
     else
-      k_refill<JS><<<g, 256, 0, c->stream>>>(in, b.wc, p.wave, c->d_radiance, js);
+      k_refill<JS><<<g, 256, 0, c->stream>>>(in, b.wc, p.wave, p.total, p.cap, c->d_radiance, js);
     kernels++;
   }
   cudaEventRecord(ev[0], c->stream);
   if (p.finish) {
-    k_finish<WIDTH, JS, ADJ><<<blocks(p.rays, 128), 128, 0, c->stream>>>(
-        in, ain, b.wc, p.wave, c->d_radiance, ADJ ? adj->g_alb : nullptr, ADJ ? adj->g_rough : nullptr, js);
+    const uint32_t lanes = finish_lanes(p.rays, p.wave);
+    k_finish<WIDTH, JS, ADJ><<<blocks(p.rays, 4u * lanes), 128, 0, c->stream>>>(
+        in, ain, b.wc, p.wave, lanes, c->d_radiance, ADJ ? adj->g_alb : nullptr, ADJ ? adj->g_rough : nullptr, js);
     kernels++;
     cudaEventRecord(ev[1], c->stream);
+    return cudaGetLastError(); /* what follows the last wave brings the counters back */
   } else {
     const unsigned g_trace = blocks(p.rays, ls.trace_block);
     const unsigned g_shade = blocks(p.rays, ls.shade_block);
@@ -1229,46 +1260,43 @@ auto wave_launcher(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, int wi
  * once every path has ended.  A wave is enqueued while the one before it runs, so its plan holds upper
  * bounds: the rays of that wave and the paths not yet started.  Once no path is left to start and at
  * most `finish_rays` rays are, the plan is k_finish's and the last.  after_last() enqueues what follows the
- * last wave; behind k_finish the GPU goes on with it while the host still waits for the counters. */
+ * last wave, and behind k_finish copies the counters to the slot it is given, so that one wait of the host
+ * covers both. */
 template <class Launch, class Last>
 nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, uint32_t finish_rays, Launch &&launch,
                            Last &&after_last, LoopStats &ls) {
-  WaveCounters *hw = static_cast<WaveCounters *>(x->h_wave); /* [0], [1]: read-back slots, [2]: upload */
-  hw[2] = WaveCounters{};
-  hw[2].total = total;
-  hw[2].cap = cap;
-  NB_CUDA(x, cudaMemcpyAsync(x->d_wave, hw + 2, sizeof(WaveCounters), cudaMemcpyHostToDevice, x->stream),
-          "upload(wave counters)");
+  WaveCounters *hw = static_cast<WaveCounters *>(x->h_wave); /* pinned read-back slots */
   /* bounds on the next wave to enqueue: its waiting rays, and the paths started before it (exact) */
   uint32_t waiting = 0, started = 0, enqueued = 0, finished = 0;
   bool finish = false;
   for (;;) {
     while (!finish && enqueued < finished + 2) {
-      WavePlan p{enqueued, 0, 0, false};
+      WavePlan p{enqueued, 0, 0, total, cap, false};
       p.rays = (uint32_t)std::min<uint64_t>(cap, (uint64_t)waiting + (total - started));
       if (p.rays == 0) break;
       p.fresh = std::min(cap, total - started);
       p.finish = finish = p.rays <= finish_rays && total - started <= cap - waiting;
       NB_CUDA(x, launch(p, ls.kernels), "wave");
       enqueued++;
-      if (finish) after_last();
+      if (finish) after_last(hw + (p.wave & 1u));
       /* at least cap - waiting of them start in this wave; how many exactly is read back */
       started += std::min(cap - waiting, total - started);
       waiting = p.rays;
     }
     const int slot = (int)(finished & 1u);
-    NB_CUDA(x, cudaEventSynchronize(x->ev_done[slot]), "waves");
+    const bool last = finish && finished + 1 == enqueued; /* k_finish: with all that is enqueued behind it */
+    NB_CUDA(x, last ? cudaStreamSynchronize(x->stream) : cudaEventSynchronize(x->ev_done[slot]), "waves");
     const cudaEvent_t *ev = x->ev_wave + 3 * slot;
     float a = 0.f, b = 0.f;
     cudaEventElapsedTime(&a, ev[0], ev[1]);
-    cudaEventElapsedTime(&b, ev[1], ev[2]);
+    if (!last) cudaEventElapsedTime(&b, ev[1], ev[2]);
     ls.t_trace += a;
     ls.t_shade += b;
     const WaveCounters r = hw[slot];
     finished++;
     auto drain = [&] { /* the wave still in flight; its counters */
       if (enqueued == finished) return cudaSuccess;
-      return cudaEventSynchronize(x->ev_done[finished & 1u]);
+      return finish ? cudaStreamSynchronize(x->stream) : cudaEventSynchronize(x->ev_done[finished & 1u]);
     };
     if (r.bad_index) { /* the device status word: stop after this wave, as the reference aborts a tile
                         * once its exception manager holds an error (integrator/Integrator.h:74-78) */
@@ -1289,7 +1317,7 @@ nova_b200_status run_waves(nova_b200_ctx *x, uint32_t total, uint32_t cap, uint3
       ls.nonfinite += r.nonfinite;
       ls.node_visits += r.node_visits;
       ls.tri_tests += r.tri_tests;
-      if (!finish) after_last();
+      if (!finish) after_last(nullptr);
       return NOVA_B200_SUCCESS;
     }
     if (!finish && x->cancel.load()) { /* nova_b200_cancel: let the wave in flight finish, enqueue nothing
@@ -1590,7 +1618,7 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
       std::copy(hj.begin(), hj.begin() + chunk.size(), many.j);
     }
     /* the chunk's samples into its films, enqueued behind its last wave */
-    auto resolve = [&] {
+    auto resolve = [&](WaveCounters *back) {
       for (size_t k = 0; k < chunk.size(); k++) {
         const Piece &P = chunk[k];
         nova_b200_ctx *c = P.ctx;
@@ -1600,14 +1628,15 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
         k_resolve<<<(NP + 255) / 256, 256, 0, x->stream>>>(
             x->d_radiance + hj[k].path_begin, NP, P.count, c->d_film_acc, c->film_clear, (float)c->film_samples,
             last_chunk[j] == ci ? film_target(j) : c->d_film_out, P.f->width, P.f->height, P.f->vertical_invert,
-            static_cast<const WaveCounters *>(x->d_wave));
+            static_cast<const WaveCounters *>(x->d_wave), k == 0 ? back : nullptr);
         c->film_clear = false;
         sum.kernels++;
       }
+      if (ci + 1 == nc) cudaEventRecord(x->ev_end, x->stream);
     };
     if (ls.trace_mode == 3) { /* the persistent wavefront: one launch runs every wave of the chunk */
       st = single ? run_persistent_w(x, one, ls, width, pb, cap, loop) : run_persistent_w(x, many, ls, width, pb, cap, loop);
-      if (st == NOVA_B200_SUCCESS) resolve();
+      if (st == NOVA_B200_SUCCESS) resolve(nullptr);
     } else {
       std::vector<std::pair<uint64_t, bool>> film_state; /* for a failure found after the resolves are enqueued */
       for (const Piece &P : chunk) film_state.emplace_back(P.ctx->film_samples, P.ctx->film_clear);
@@ -1629,7 +1658,6 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
     }
   }
   NB_CUDA(x, cudaGetLastError(), "render kernels");
-  NB_CUDA(x, cudaEventRecord(x->ev_end, x->stream), "event");
   for (size_t j = 0; j < nj; j++)
     if (!early[j] && (st = copy_film(j, x->stream)) != NOVA_B200_SUCCESS) return st;
   NB_CUDA(x, cudaStreamSynchronize(x->stream), "render");
@@ -1839,11 +1867,14 @@ nova_b200_status nb_backward(nova_b200_ctx *c, const nova_b200_frame *f, const f
     J.path_begin = 0;
     J.n_paths = NP * take;
     /* primal: each path's radiance into the radiance buffer */
+    auto read_back = [&](WaveCounters *back) {
+      if (back) cudaMemcpyAsync(back, c->d_wave, sizeof(WaveCounters), cudaMemcpyDeviceToHost, c->stream);
+    };
     if (!reuse &&
-        (st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher(c, one, ls, width), [] {}, primal)) != NOVA_B200_SUCCESS)
+        (st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher(c, one, ls, width), read_back, primal)) != NOVA_B200_SUCCESS)
       return st;
     /* replay with the adjoint */
-    if ((st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher<true>(c, one, ls, width, &adj), [] {}, replay)) !=
+    if ((st = run_waves(c, J.n_paths, cap, ls.finish_rays, wave_launcher<true>(c, one, ls, width, &adj), read_back, replay)) !=
         NOVA_B200_SUCCESS)
       return st;
     sum.paths += J.n_paths;
