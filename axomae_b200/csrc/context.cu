@@ -223,7 +223,9 @@ void free_scene(nova_b200_ctx *c) {
   if (c->d_tris) cudaFreeAsync(c->d_tris, c->stream);
   if (c->d_valid) cudaFreeAsync(c->d_valid, c->stream);
   if (c->d_blas_root) cudaFreeAsync(c->d_blas_root, c->stream);
+  if (c->d_inst_rec) cudaFreeAsync(c->d_inst_rec, c->stream);
   c->d_blas_root = nullptr;
+  c->d_inst_rec = nullptr;
   c->h_meshes.clear();
   c->d_arena = nullptr;
   c->d_nodes = nullptr;
@@ -474,6 +476,16 @@ __global__ void k_relocate(float4 *nodes, uint32_t n_nodes, uint32_t node_base, 
   n3.y = __int_as_float(r[1]);
 }
 
+/* What a walk reads to enter an instance (DevScene::inst_rec). */
+__global__ void k_instance_records(const nb::DevInstance *inst, uint32_t n, const uint32_t *blas_root, float4 *rec) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const nb::DevInstance &I = inst[i];
+  for (int r = 0; r < 3; r++) rec[4 * (size_t)i + r] = make_float4(I.inv[r], I.inv[4 + r], I.inv[8 + r], I.inv[12 + r]);
+  rec[4 * (size_t)i + 3] = make_float4(__uint_as_float(blas_root[I.mesh]), __uint_as_float(I.prim_offset),
+                                       I.identity ? 1.f : 0.f, 0.f);
+}
+
 /* World box of each instance: the eight corners of its mesh's bottom-level root box, transformed. */
 __global__ void k_instance_boxes(const nb::DevInstance *inst, uint32_t n, const float4 *nodes, const uint32_t *blas_root,
                                  float4 *lo, float4 *hi) {
@@ -578,6 +590,7 @@ nova_b200_status build_two_level(nova_b200_ctx *c, const nb::BvhBuildParams &p, 
   cudaError_t e = cudaMallocAsync(&c->d_nodes, sizeof(float4) * 4 * total_nodes, c->stream);
   if (e == cudaSuccess) e = cudaMallocAsync(&c->d_tris, sizeof(float4) * (nb::kTriStride * total_tris + nb::kTriPad), c->stream);
   if (e == cudaSuccess) e = cudaMallocAsync(&c->d_blas_root, sizeof(uint32_t) * n_meshes, c->stream);
+  if (e == cudaSuccess) e = cudaMallocAsync(&c->d_inst_rec, sizeof(float4) * 4 * (size_t)n_inst, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->d_nodes, 0, sizeof(float4) * 4 * total_nodes, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->d_tris, 0, sizeof(float4) * (nb::kTriStride * total_tris + nb::kTriPad), c->stream);
   if (e == cudaSuccess) e = cudaMallocAsync(&lo, sizeof(float4) * scratch, c->stream);
@@ -646,6 +659,7 @@ nova_b200_status build_two_level(nova_b200_ctx *c, const nb::BvhBuildParams &p, 
   pt.max_leaf = 1;
   pt.hard_leaf = 1;
   const nb::DevInstance *d_inst = c->scene.instances;
+  k_instance_records<<<(n_inst + 255) / 256, 256, 0, c->stream>>>(d_inst, n_inst, c->d_blas_root, c->d_inst_rec);
   k_instance_boxes<<<(n_inst + 255) / 256, 256, 0, c->stream>>>(d_inst, n_inst, c->d_nodes, c->d_blas_root, lo, hi);
   e = nb::build_bvh(lo, hi, n_inst, pt, c->d_nodes, order, c->stream, &r);
   if (e == cudaSuccess) {
@@ -993,10 +1007,12 @@ nova_b200_status nova_b200_build_bvh(nova_b200_ctx *c, const nova_b200_bvh_optio
   if (c->d_nodes) cudaFreeAsync(c->d_nodes, c->stream);
   if (c->d_tris) cudaFreeAsync(c->d_tris, c->stream);
   if (c->d_blas_root) cudaFreeAsync(c->d_blas_root, c->stream);
+  if (c->d_inst_rec) cudaFreeAsync(c->d_inst_rec, c->stream);
   c->d_nodes = nullptr;
   c->d_tris = nullptr;
   c->d_blas_root = nullptr;
-  c->scene.blas_root = nullptr;
+  c->d_inst_rec = nullptr;
+  c->scene.inst_rec = nullptr;
   c->bvh_ready = false;
   c->primal_valid = false;
   if (width == 1) {
@@ -1005,7 +1021,7 @@ nova_b200_status nova_b200_build_bvh(nova_b200_ctx *c, const nova_b200_bvh_optio
     if (st != NOVA_B200_SUCCESS) return st;
     c->scene.nodes = c->d_nodes;
     c->scene.tris = c->d_tris;
-    c->scene.blas_root = c->d_blas_root;
+    c->scene.inst_rec = c->d_inst_rec;
     c->scene.width = 1;
     c->bvh_width = 1;
     c->n_nodes = r.n_nodes;

@@ -29,6 +29,7 @@ struct nova_b200_ctx {
   std::vector<nb::DevInstance> h_instances;
   std::vector<nb::DevMesh> h_meshes;      /* device pointers, host copy of the mesh table */
   uint32_t *d_blas_root = nullptr;        /* two-level BVH: per mesh, its bottom-level root node */
+  float4 *d_inst_rec = nullptr;           /* two-level BVH: per instance, what a walk reads to enter it */
   uint32_t *d_valid = nullptr;   /* global primitive ids that can be hit, ascending (device) */
   uint32_t n_valid = 0;
   uint64_t n_prims = 0;

@@ -81,7 +81,8 @@ struct DevScene {
   uint32_t has_emissive;
   const float *diff_albedo;  /* differentiable parameters (NULL: textures): 3 x n_prims RGB albedo */
   const float *diff_rough;   /* and n_materials roughness values */
-  const uint32_t *blas_root; /* two-level BVH (width 1): per mesh, the node index of its bottom-level root */
+  const float4 *inst_rec;    /* two-level BVH (width 1): per instance 64 B, the rows of its inverse transform,
+                              * then (its mesh's root node, its first primitive id, 1 if it is the identity, 0) */
 };
 
 constexpr int kAcosPrecision = 500000;

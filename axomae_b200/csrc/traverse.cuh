@@ -434,24 +434,28 @@ NB_D TraceResult trace_closest_tl(const DevScene &sc, V3 o, V3 d, uint64_t *node
   uint32_t nv = 0, tt = 0;
   for (;;) {
     const bool inner = cur >= 0;
-    if (!inner && !inside) { /* top-level leaf: enter the instance */
-      const DevInstance &I = sc.instances[leaf_first(cur)];
-      if (!I.identity) {
-        ro = xform_point(I.inv, o);
-        rd = xform_dir(I.inv, d);
-        sr.set(ro, rd);
-      }
-      prim_base = I.prim_offset;
-      inst_in = leaf_first(cur);
-      inside = true;
-      if (sp < kTraversalStack) stack[sp++] = kLeaveInstance;
-      cur = (int32_t)sc.blas_root[I.mesh];
-      continue;
-    }
-    const Rec q = load_rec(inner ? sc.nodes + 4 * (size_t)(uint32_t)cur : sc.tris + kTriStride * (size_t)leaf_first(cur));
+    const Rec q = load_rec(inner    ? sc.nodes + 4 * (size_t)(uint32_t)cur
+                           : inside ? sc.tris + kTriStride * (size_t)leaf_first(cur)
+                                    : sc.inst_rec + 4 * (size_t)leaf_first(cur));
     if (inner) {
       nv++;
       if (visit_inner(q, sr, tmax, stack, sp, cur)) continue;
+    } else if (!inside) { /* top-level leaf: enter the instance */
+      if (q.q3.z == 0.f) { /* xform_point and xform_dir on the inverse's rows */
+        ro = V3{(q.q0.x * o.x + q.q0.y * o.y) + (q.q0.z * o.z + q.q0.w * 1.f),
+                (q.q1.x * o.x + q.q1.y * o.y) + (q.q1.z * o.z + q.q1.w * 1.f),
+                (q.q2.x * o.x + q.q2.y * o.y) + (q.q2.z * o.z + q.q2.w * 1.f)};
+        rd = V3{(q.q0.x * d.x + q.q0.y * d.y) + (q.q0.z * d.z + q.q0.w * 0.f),
+                (q.q1.x * d.x + q.q1.y * d.y) + (q.q1.z * d.z + q.q1.w * 0.f),
+                (q.q2.x * d.x + q.q2.y * d.y) + (q.q2.z * d.z + q.q2.w * 0.f)};
+        sr.set(ro, rd);
+      }
+      prim_base = __float_as_uint(q.q3.y);
+      inst_in = leaf_first(cur);
+      inside = true;
+      if (sp < kTraversalStack) stack[sp++] = kLeaveInstance;
+      cur = __float_as_int(q.q3.x);
+      continue;
     } else { /* bottom-level leaf: object-space triangles, mesh-local ids */
       tt++;
       float ht, hu, hv;
@@ -502,17 +506,17 @@ NB_D TraceResult trace_closest_w(const DevScene &sc, V3 o, V3 d, uint64_t *node_
 struct WalkTables {
   const float4 *nodes, *tris;
   const DevInstance *instances;
-  const uint32_t *blas_root;
+  const float4 *inst_rec;
 };
 template <int WIDTH>
 __device__ __noinline__ TraceResult walk_tables(WalkTables w, V3 o, V3 d) {
   DevScene sc;
-  sc.nodes = w.nodes, sc.tris = w.tris, sc.instances = w.instances, sc.blas_root = w.blas_root;
+  sc.nodes = w.nodes, sc.tris = w.tris, sc.instances = w.instances, sc.inst_rec = w.inst_rec;
   return trace_closest_w<WIDTH>(sc, o, d);
 }
 template <int WIDTH>
 NB_D TraceResult walk(const DevScene &sc, V3 o, V3 d) {
-  return walk_tables<WIDTH>(WalkTables{sc.nodes, sc.tris, sc.instances, sc.blas_root}, o, d);
+  return walk_tables<WIDTH>(WalkTables{sc.nodes, sc.tris, sc.instances, sc.inst_rec}, o, d);
 }
 
 /* The same on the scene's own width. */
