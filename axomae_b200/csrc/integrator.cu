@@ -53,7 +53,11 @@ namespace {
 using namespace nb;
 
 constexpr uint32_t kQueueCapDefault = 1u << 23; /* rays per wave unless tuned */
-constexpr size_t kRadianceCapBytes = 4ull << 30;
+/* Radiance buffer: all of a call's paths up to kRadianceCapBytes, else chunks of kRadianceChunkBytes.  Nothing
+ * reuses a chunked call's radiance, so its chunks need only be long against their drain (0.35 ms each): 2^31
+ * paths took 294 ms in chunks of 4 GiB, 297 in 2, 303 in 1, 307 in 0.75 and 315 in 0.5 GiB (307 in chunks of
+ * 4 GiB before the waves were made shorter), and 0.75 GiB leaves the rest to the other contexts on the GPU. */
+constexpr size_t kRadianceCapBytes = 4ull << 30, kRadianceChunkBytes = 768ull << 20;
 constexpr unsigned kRRDimBase = 200; /* Russian roulette decisions use Sobol dimension 200 + bounce */
 constexpr int kMaxDepth = 48;        /* 2 + 4 (depth + 1) Sobol dimensions must stay below 200 */
 
@@ -333,8 +337,8 @@ __device__ __forceinline__ unsigned warp_append(bool flag, unsigned *counter) {
 /* Resident blocks of 128 threads per SM that k_trace is compiled for (the register bound is
  * 65536 / (128 * blocks)).  Binary: 10 blocks (48 registers, next to no spills), 21.6 ms of traversal
  * on an 8-frame batch against 22.3 at 9 and 23.4 at 8.  Two-level: the walk also holds the world ray
- * and the instance, so 10 blocks spill 150 B a thread: 5.3 ms on 1000 instances at 720p, 9 blocks
- * (56 registers) 3.7 ms, 8 blocks 3.8. */
+ * and the instance, so 10 blocks spill: 3.84 ms on 1000 instances at 720p, 9 blocks (56 registers) 3.64,
+ * 8 blocks 3.61. */
 template <int WIDTH>
 constexpr int kTraceBlocks = WIDTH == 1 ? 9 : 10;
 
@@ -1478,8 +1482,8 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
     max_np = std::max(max_np, np);
     total += np * (uint64_t)frames[j]->sample_count;
   }
-  const uint64_t cap_entries = kRadianceCapBytes / sizeof(float4);
-  const uint64_t radiance = std::max<uint64_t>(max_np, std::min<uint64_t>(total, cap_entries));
+  const uint64_t radiance = std::max<uint64_t>(
+      max_np, (total <= kRadianceCapBytes / sizeof(float4)) ? total : kRadianceChunkBytes / sizeof(float4));
   const nova_b200_tuning &tu = x->tuning;
   const uint32_t qc = tu.queue_capacity ? tu.queue_capacity : kQueueCapDefault;
   const uint32_t cap = (uint32_t)std::min<uint64_t>(qc, std::max<uint64_t>(radiance, 1024));
