@@ -16,9 +16,12 @@
  *                    stbi_loadf in IO::Loader::loadRadianceFile, sources/IO/Loader_image.cpp:50-62,
  *                    146-192; stb is an un-vendored submodule of the reference, github.com/nothings/stb).
  *
- * Host code: the file's text header and its run-length scanline packets, serial byte work on a
- * buffer of 4 bytes per pixel (the device encodes, the host only packs).
+ *   k_rle_find, k_rle_walk, k_rle_link, k_rle_rows  where the rows of a run-length file start, and their
+ *                    packets expanded.
+ *
+ * Host code: the file's text header, and the packet walk of small or irregular run-length files.
  */
+#include <climits>
 #include <cstring>
 #include <fstream>
 #include <string>
@@ -180,8 +183,9 @@ __device__ __forceinline__ float4 rgbe_decode(uint32_t word) {
 }
 
 /* Four pixels per thread: one 16-byte load of RGBE words, four float4 stores (both buffers 16-byte
- * aligned); the last thread takes the ragged end pixel by pixel. */
-__global__ void k_rgbe_decode(const uint32_t *src, uint64_t n, float4 *dst) {
+ * aligned); the last thread takes the ragged end pixel by pixel.  ok: null, or 0 for "nothing to decode". */
+__global__ void k_rgbe_decode(const uint32_t *src, uint64_t n, float4 *dst, const uint32_t *ok) {
+  if (ok && *ok == 0u) return;
   const uint64_t i4 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 + 4 <= n) {
     const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src + i4));
@@ -331,6 +335,214 @@ __global__ void k_rle_unpack(const unsigned char *body, const uint64_t *starts, 
   }
 }
 
+/* A run-length file's rows on the device.  Where a row starts is known only when the one before has been
+ * walked, so every byte position that holds the row header (2, 2, width >> 8, width & 255) is walked as a
+ * row (k_rle_find, k_rle_walk; a few of them are packet data), and k_rle_link follows the ends from the
+ * first to the last row.  A chain that does not close (a cut or damaged file, a flat one) clears the status
+ * word: the host then reads the file again, as it reads small ones. */
+
+/* Two kernels: WRITE = false counts a block's matches, WRITE = true places the first `most` of them in file
+ * order.  `chunk` (bytes per block) is a multiple of a tile, 16 bytes a thread; the body is padded by 256
+ * zeros.  Bound by the body's bytes. */
+constexpr int kFindThreads = 256, kFindTile = 16 * kFindThreads, kFindBlocks = 2048;
+
+template <bool WRITE>
+__global__ void __launch_bounds__(kFindThreads)
+    k_rle_find(const unsigned char *body, uint32_t n, uint32_t pattern, uint32_t chunk, uint32_t *counts, uint32_t most,
+               uint32_t *starts) {
+  __shared__ uint32_t warp_sum[kFindThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  /* exclusive prefix of v over the block and the block's total */
+  auto scan = [&](uint32_t v, uint32_t &total) {
+    uint32_t x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) warp_sum[w] = x;
+    __syncthreads();
+    uint32_t before = 0;
+    total = 0;
+    for (int k = 0; k < kFindThreads / 32; k++) {
+      const uint32_t t = warp_sum[k];
+      if (k < w) before += t;
+      total += t;
+    }
+    return before + x - v;
+  };
+  uint32_t base = 0, found = 0, total;
+  if (WRITE) {
+    uint32_t mine = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kFindThreads) mine += counts[b];
+    scan(mine, base);
+    if (base >= most || counts[blockIdx.x] == 0u) return;
+  }
+  const uint64_t first = (uint64_t)blockIdx.x * chunk, last = min((uint64_t)n, first + chunk);
+  for (uint64_t tile = first; tile < last; tile += kFindTile) {
+    const uint64_t p = tile + 16u * threadIdx.x;
+    uint32_t match = 0;
+    if (p < n) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4 *>(body + p));
+      const uint32_t v[5] = {q.x, q.y, q.z, q.w, __ldg(reinterpret_cast<const uint32_t *>(body + p + 16))};
+#pragma unroll
+      for (int k = 0; k < 16; k++)
+        if (__funnelshift_r(v[k >> 2], v[(k >> 2) + 1], 8 * (k & 3)) == pattern && p + k + 4 <= n) match |= 1u << k;
+    }
+    if (!WRITE) {
+      found += __popc(match);
+    } else {
+      uint32_t at = base + scan(__popc(match), total);
+      for (; match; match &= match - 1u, at++)
+        if (at < most) starts[at] = (uint32_t)p + __ffs(match) - 1u;
+      base += total;
+    }
+  }
+  if (!WRITE) {
+    scan(found, total);
+    if (threadIdx.x == 0) counts[blockIdx.x] = total;
+  }
+}
+
+/* The bytes [start, start + bytes) of the body to shared memory by the whole block, 16 at a time; the first
+ * of them lands at start & 15. */
+__device__ __forceinline__ void stage_row(const unsigned char *body, uint32_t start, uint32_t bytes, uint4 *staged) {
+  const uint4 *src = reinterpret_cast<const uint4 *>(body + (start & ~15u));
+  for (uint32_t i = threadIdx.x; 16u * i < (start & 15u) + bytes; i += blockDim.x) staged[i] = __ldg(src + i);
+  __syncthreads();
+}
+
+/* One block per position placed (0xffffffff: none): its row's bytes (2 per value at most) into shared
+ * memory, then one thread walks the packet headers of the four planes, which follow one another: where each
+ * plane starts and the row ends, in `walked`; an end of 0 when this is no row. */
+struct WalkedRow {
+  uint32_t plane[4], end;
+};
+__global__ void __launch_bounds__(128) k_rle_walk(const unsigned char *body, uint32_t n, const uint32_t *starts, int w,
+                                                  uint32_t cap, WalkedRow *walked) {
+  extern __shared__ uint4 staged[];
+  const uint32_t start = starts[blockIdx.x];
+  if (start == 0xffffffffu) return;
+  const uint32_t shift = start & 15u, bytes = min(min(n - start, 8u * (uint32_t)w + 4u), cap - shift);
+  stage_row(body, start, bytes, staged);
+  if (threadIdx.x != 0) return;
+  const unsigned char *sm = reinterpret_cast<const unsigned char *>(staged) + shift;
+  WalkedRow r;
+  uint32_t p = 4u;
+  bool fine = true;
+  for (int k = 0; k < 4; k++) {
+    r.plane[k] = p;
+    for (uint32_t left = (uint32_t)w; fine && left > 0u;) {
+      const uint32_t head = p < bytes ? sm[p] : 0u, cnt = head > 128u ? head - 128u : head;
+      fine = cnt != 0u && cnt <= left;
+      p += head > 128u ? 2u : 1u + cnt;
+      left -= cnt;
+    }
+  }
+  r.end = fine && p <= bytes ? start + p : 0u;
+  walked[blockIdx.x] = r;
+}
+
+/* Which of the walked positions are the image's h rows: the first, and each one that starts where the row
+ * before ends.  One block; without matches in packet data position j is row j, which all threads check at
+ * once, else one warp follows the links, 32 positions in its lanes.  *ok becomes 0 when the rows do not chain. */
+__global__ void __launch_bounds__(1024) k_rle_link(const uint32_t *starts, const WalkedRow *walked, uint32_t most,
+                                                   uint32_t h, uint32_t *next, uint32_t *rows, uint32_t *ok) {
+  constexpr uint32_t kNone = 0xffffffffu;
+  bool plain = true;
+  for (uint32_t i = threadIdx.x; i < most && starts[i] != kNone; i += blockDim.x) {
+    const uint32_t end = walked[i].end;
+    uint32_t to = kNone;
+    if (end != 0u && i + 1u < most) {
+      uint32_t lo = i + 1u, hi = most; /* the first position at or after the end (0xffffffff: past the last) */
+      if (starts[lo] < end)
+        while (lo < hi) {
+          const uint32_t mid = lo + (hi - lo) / 2u;
+          if (starts[mid] < end)
+            lo = mid + 1u;
+          else
+            hi = mid;
+        }
+      if (lo < most && starts[lo] == end) to = lo;
+    }
+    next[i] = to;
+    if (i < h) {
+      rows[i] = i;
+      plain = plain && (i + 1u < h ? to == i + 1u : end != 0u);
+    }
+  }
+  if (__syncthreads_and(plain && (h <= most && starts[h - 1u] != kNone))) return;
+  if (threadIdx.x >= 32u) return;
+  uint32_t at = 0, mine = 0, base = kNone;
+  for (uint32_t j = 0; j < h; j++) {
+    if (base == kNone || at - base >= 32u) {
+      base = at;
+      mine = at + threadIdx.x < most && starts[at + threadIdx.x] != kNone ? next[at + threadIdx.x] : kNone;
+    }
+    if (threadIdx.x == 0) rows[j] = at;
+    if (j + 1u == h) {
+      if (threadIdx.x == 0 && walked[at].end == 0u) *ok = 0u;
+      return;
+    }
+    at = __shfl_sync(0xffffffffu, mine, at - base);
+    if (at == kNone) {
+      if (threadIdx.x == 0) *ok = 0u;
+      return;
+    }
+  }
+}
+
+/* Run-length expansion of the linked rows, one block per row: its bytes into shared memory, then one warp per
+ * plane walks 32 packets, one to a lane, and writes their values: packet by packet when they are long, else 32
+ * values at a time, each lane finding its packet by bisection over the lanes (exponents come in packets of a
+ * few values: packet by packet they took 44 us).  1024 x 512 of random values, 118,000 packets in 2 MB: 21 us (the walk before it 17). */
+__global__ void __launch_bounds__(128) k_rle_rows(const unsigned char *body, const uint32_t *starts,
+                                                  const WalkedRow *walked, const uint32_t *rows, int w,
+                                                  unsigned char *rgbe, const uint32_t *ok) {
+  extern __shared__ uint4 staged[];
+  if (*ok == 0u) return;
+  const uint32_t i = rows[blockIdx.x], start = starts[i];
+  const WalkedRow &r = walked[i];
+  stage_row(body, start, r.end - start, staged);
+  const unsigned char *sm = reinterpret_cast<const unsigned char *>(staged) + (start & 15u);
+  const int lane = threadIdx.x & 31, plane = threadIdx.x >> 5;
+  unsigned char *o = rgbe + (size_t)blockIdx.x * w * 4 + plane;
+  uint32_t p = r.plane[plane];
+  for (int x = 0; x < w;) {
+    const int x0 = x;
+    int first = INT_MAX; /* the lane's packet: its first value, and where its bytes are (a run's: bit 31) */
+    uint32_t src = 0;
+    int packets = 0;
+    for (; packets < 32 && x < w; packets++) {
+      const uint32_t head = sm[p];
+      const bool run = head > 128u;
+      const uint32_t cnt = run ? head - 128u : head;
+      if (lane == packets) first = x, src = (p + 1u) | (run ? 0x80000000u : 0u);
+      p += run ? 2u : 1u + cnt;
+      x += (int)cnt;
+    }
+    if (x - x0 >= 32 * packets) { /* long packets: one after the other */
+      for (int k = 0; k < packets; k++) {
+        const uint32_t from = __shfl_sync(0xffffffffu, src, k);
+        const int at = __shfl_sync(0xffffffffu, first, k);
+        const int end = k + 1 < packets ? __shfl_sync(0xffffffffu, first, k + 1) : x;
+        for (int t = at + lane; t < end; t += 32)
+          o[4 * (size_t)t] = sm[(from & 0x7fffffffu) + (from >> 31 ? 0u : (uint32_t)(t - at))];
+      }
+      continue;
+    }
+    for (int b = x0; b < x; b += 32) {
+      const int t = b + lane;
+      int l = 0; /* the last packet that starts at or before t */
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, first, l + step) <= t) l += step;
+      const uint32_t from = __shfl_sync(0xffffffffu, src, l);
+      const int at = __shfl_sync(0xffffffffu, first, l);
+      if (t < x) o[4 * (size_t)t] = sm[(from & 0x7fffffffu) + (from >> 31 ? 0u : (uint32_t)(t - at))];
+    }
+  }
+}
+
 /* ---- host: the file format ----------------------------------------------------------------- */
 
 constexpr int kMaxDim = 1 << 24; /* the largest width / height the loader accepts */
@@ -454,21 +666,138 @@ nova_b200_status scan_rows(nova_b200_ctx *c, const std::vector<unsigned char> &b
   return NOVA_B200_SUCCESS;
 }
 
-/* The file, or its first `limit` bytes (limit 0: all); *whole tells whether all of it was read. */
-nova_b200_status read_file(nova_b200_ctx *c, const char *path, std::vector<unsigned char> &bytes, size_t limit = 0,
-                           bool *whole = nullptr) {
+/* Opens a file, unbuffered (it is read in large pieces), and reads the first `limit` bytes of its `size`. */
+nova_b200_status read_head(nova_b200_ctx *c, const char *path, std::ifstream &f, size_t limit,
+                           std::vector<unsigned char> &bytes, size_t &size) {
   using namespace nbctx;
   if (!path) return fail(c, NOVA_B200_INVALID_ARGUMENT, "path is null%s");
-  std::ifstream f(path, std::ios::binary | std::ios::ate);
+  f.rdbuf()->pubsetbuf(nullptr, 0);
+  f.open(path, std::ios::binary | std::ios::ate);
   if (!f) return fail(c, NOVA_B200_INVALID_ARGUMENT, "cannot open %s", path);
-  const std::streamoff size = f.tellg();
-  if (size < 0) return fail(c, NOVA_B200_INVALID_ARGUMENT, "cannot read %s", path);
-  const size_t n = limit ? std::min((size_t)size, limit) : (size_t)size;
-  bytes.resize(n);
+  const std::streamoff end = f.tellg();
+  if (end < 0) return fail(c, NOVA_B200_INVALID_ARGUMENT, "cannot read %s", path);
+  size = (size_t)end;
+  bytes.resize(std::min(size, limit));
   f.seekg(0);
-  if (n && !f.read(reinterpret_cast<char *>(bytes.data()), (std::streamsize)n))
+  if (!bytes.empty() && !f.read(reinterpret_cast<char *>(bytes.data()), (std::streamsize)bytes.size()))
     return fail(c, NOVA_B200_INVALID_ARGUMENT, "cannot read %s", path);
-  if (whole) *whole = n == (size_t)size;
+  return NOVA_B200_SUCCESS;
+}
+
+/* The rest of a file whose head is in `bytes`. */
+nova_b200_status read_rest(nova_b200_ctx *c, const char *path, std::ifstream &f, std::vector<unsigned char> &bytes,
+                           size_t size) {
+  const size_t have = bytes.size();
+  if (size <= have) return NOVA_B200_SUCCESS;
+  bytes.resize(size);
+  f.clear();
+  f.seekg((std::streamoff)have);
+  if (!f.read(reinterpret_cast<char *>(bytes.data() + have), (std::streamsize)(size - have)))
+    return nbctx::fail(c, NOVA_B200_INVALID_ARGUMENT, "cannot read %s", path);
+  return NOVA_B200_SUCCESS;
+}
+
+nova_b200_status check_read(nova_b200_ctx *c, const Header &hd, const float *rgba_device, uint64_t capacity) {
+  using namespace nbctx;
+  const uint64_t npx = (uint64_t)hd.w * hd.h;
+  if (npx > (1ull << 31)) return fail(c, NOVA_B200_INVALID_ARGUMENT, "HDR image larger than 2^31 pixels%s");
+  if (capacity < npx * 4) return fail(c, NOVA_B200_INVALID_ARGUMENT, "output holds fewer than width * height * 4 floats%s");
+  if (rgba_device && (reinterpret_cast<uintptr_t>(rgba_device) & 15))
+    return fail(c, NOVA_B200_INVALID_ARGUMENT, "rgba_device must be 16-byte aligned%s");
+  return NOVA_B200_SUCCESS;
+}
+
+/* hdr_read of a run-length file of more than kDeviceBytes or kDevicePixels: the bytes go through the context's pinned staging to
+ * the device as they are read, and the device finds, checks and expands the rows.  *done stays false when
+ * this is no such file, or one whose rows it could not chain: nothing has been written then, and the
+ * caller reads the file the other way, which also says what is wrong with it.
+ *
+ * The other way's walk of the packets on the host costs 2.5 ns a packet, this one five short kernels and their
+ * gaps.  Random values (few packets a byte): 78 KB 75 us the other way and 102 this way, 256 KB 107 and 116,
+ * 513 KB 153 and 126, 2 MB 550 and 271, 32 MB 8.4 and 3.0 ms; one colour (66 values a byte, so the pixels
+ * tell): 0.5 Mpixel 81 and 92, 2 Mpixel 160 and 120, 8 Mpixel 450 and 240. */
+constexpr size_t kHeadBytes = 1 << 16, kFilePiece = 1 << 18, kRowSmem = 200 << 10;
+constexpr size_t kDeviceBytes = 5 << 16, kDevicePixels = 1 << 20;
+
+nova_b200_status read_rows_on_device(nova_b200_ctx *c, std::ifstream &f, const std::vector<unsigned char> &head,
+                                     size_t size, float *rgba_host, float *rgba_device, uint64_t capacity, bool *done) {
+  using namespace nbctx;
+  *done = false;
+  if (size <= head.size()) return NOVA_B200_SUCCESS; /* the head is all of it */
+  Header hd;
+  if (parse_header(c, head, hd) || hd.data + 4 > head.size() || !rle_width(hd.w)) return NOVA_B200_SUCCESS;
+  const uint32_t pattern = 2u | 2u << 8 | (uint32_t)(hd.w >> 8) << 16 | (uint32_t)(hd.w & 255) << 24;
+  uint32_t word;
+  std::memcpy(&word, &head[hd.data], 4);
+  const uint64_t n = size - hd.data;
+  if (n <= kDeviceBytes && (uint64_t)hd.w * hd.h < kDevicePixels) return NOVA_B200_SUCCESS;
+  if (word != pattern || n >= 0xffffffffull || n < 4ull * (uint64_t)hd.h) return NOVA_B200_SUCCESS;
+  nova_b200_status st = check_read(c, hd, rgba_device, capacity);
+  if (st) return st;
+  cudaSetDevice(c->device);
+  if ((st = nb_ensure_stage(c, 4 * kFilePiece))) return st;
+  const uint64_t npx = (uint64_t)hd.w * hd.h;
+  const uint32_t h = (uint32_t)hd.h;
+  const uint64_t tiles = (n + kFindTile - 1) / kFindTile, per = (tiles + kFindBlocks - 1) / kFindBlocks;
+  const uint32_t chunk = (uint32_t)(per * kFindTile), blocks = (uint32_t)((tiles + per - 1) / per);
+  const uint32_t cap = (uint32_t)std::min<size_t>((8 * (size_t)hd.w + 4 + 15 + 15) & ~(size_t)15, kRowSmem);
+  unsigned char *d_body = nullptr, *d_rgbe = nullptr;
+  /* positions taken for rows; packet data that looks like one is rare, and the rest is left to the host */
+  const uint32_t most = (uint32_t)std::min<uint64_t>((uint64_t)h + h / 2 + 1024, n / 4);
+  WalkedRow *d_walked = nullptr;
+  uint32_t *d_ok = nullptr;
+  float4 *d_out = reinterpret_cast<float4 *>(rgba_device), *tmp = nullptr;
+  cudaError_t e = cudaMallocAsync(&d_body, n + 256, c->stream);
+  if (e == cudaSuccess) e = cudaMallocAsync(&d_rgbe, npx * 4, c->stream);
+  if (e == cudaSuccess) e = cudaMallocAsync(&d_walked, sizeof(WalkedRow) * most, c->stream);
+  if (e == cudaSuccess) e = cudaMallocAsync(&d_ok, sizeof(uint32_t) * (1 + 2 * (size_t)most + h + blocks), c->stream);
+  uint32_t *d_starts = d_ok + 1, *d_next = d_starts + most, *d_rows = d_next + most, *d_counts = d_rows + h;
+  if (e == cudaSuccess && !d_out) {
+    e = cudaMallocAsync(&tmp, npx * sizeof(float4), c->stream);
+    d_out = tmp;
+  }
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_body + n, 0, 256, c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_ok, 0xff, sizeof(uint32_t) * (1 + (size_t)most), c->stream);
+  bool read = true;
+  f.seekg((std::streamoff)hd.data);
+  const size_t slots = c->h_stage_bytes / kFilePiece;
+  for (uint64_t off = 0, k = 0; e == cudaSuccess && read && off < n; off += kFilePiece, k++) {
+    if (k % slots == 0) e = cudaStreamSynchronize(c->stream); /* the copies out of the staging are done */
+    char *piece = static_cast<char *>(c->h_stage) + (k % slots) * kFilePiece;
+    const size_t bytes = (size_t)std::min<uint64_t>(kFilePiece, n - off);
+    read = (bool)f.read(piece, (std::streamsize)bytes);
+    if (e == cudaSuccess && read) e = cudaMemcpyAsync(d_body + off, piece, bytes, cudaMemcpyHostToDevice, c->stream);
+  }
+  uint32_t ok = 0;
+  if (e == cudaSuccess && read) {
+    cudaEventRecord(c->ev_begin, c->stream);
+    const unsigned char *body = d_body;
+    k_rle_find<false><<<blocks, kFindThreads, 0, c->stream>>>(body, (uint32_t)n, pattern, chunk, d_counts, most, d_starts);
+    k_rle_find<true><<<blocks, kFindThreads, 0, c->stream>>>(body, (uint32_t)n, pattern, chunk, d_counts, most, d_starts);
+    for (const void *kernel : {(const void *)k_rle_walk, (const void *)k_rle_rows})
+      if (cap > 48 << 10 && e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem);
+    if (e == cudaSuccess) {
+      k_rle_walk<<<most, 128, cap, c->stream>>>(body, (uint32_t)n, d_starts, hd.w, cap, d_walked);
+      k_rle_link<<<1, 1024, 0, c->stream>>>(d_starts, d_walked, most, h, d_next, d_rows, d_ok);
+      k_rle_rows<<<h, 128, cap, c->stream>>>(body, d_starts, d_walked, d_rows, hd.w, d_rgbe, d_ok);
+      k_rgbe_decode<<<(unsigned)((npx + 1023) / 1024), 256, 0, c->stream>>>(
+          reinterpret_cast<const uint32_t *>(d_rgbe), npx, d_out, d_ok);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    cudaEventRecord(c->ev_end, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c->h_counters, d_ok, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) ok = c->h_counters[0];
+    if (ok && rgba_host)
+      e = cudaMemcpyAsync(rgba_host, d_out, npx * sizeof(float4), cudaMemcpyDeviceToHost, c->stream);
+  }
+  for (void *ptr : {(void *)d_body, (void *)d_rgbe, (void *)d_walked, (void *)d_ok, (void *)tmp})
+    if (ptr) cudaFreeAsync(ptr, c->stream);
+  const cudaError_t synced = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) e = synced;
+  if (e != cudaSuccess) return cuda_fail(c, e, "hdr_read");
+  *done = ok != 0;
   return NOVA_B200_SUCCESS;
 }
 
@@ -537,13 +866,14 @@ extern "C" nova_b200_status nova_b200_snapshot(nova_b200_ctx *c, const float *fi
 extern "C" nova_b200_status nova_b200_hdr_info(nova_b200_ctx *c, const char *path, int32_t *width, int32_t *height) {
   /* the header from the first 64 KB; the whole file only when the header runs past them */
   std::vector<unsigned char> bytes;
-  bool whole = false;
-  nova_b200_status st = read_file(c, path, bytes, 65536, &whole);
+  std::ifstream f;
+  size_t size = 0;
+  nova_b200_status st = read_head(c, path, f, kHeadBytes, bytes, size);
   if (st) return st;
   Header hd;
   st = parse_header(c, bytes, hd);
-  if (!whole && (st || hd.data >= bytes.size())) {
-    if ((st = read_file(c, path, bytes))) return st;
+  if (bytes.size() < size && (st || hd.data >= bytes.size())) {
+    if ((st = read_rest(c, path, f, bytes, size))) return st;
     st = parse_header(c, bytes, hd);
   }
   if (st) return st;
@@ -556,16 +886,19 @@ extern "C" nova_b200_status nova_b200_hdr_read(nova_b200_ctx *c, const char *pat
                                                float *rgba_device, uint64_t capacity) {
   using namespace nbctx;
   if (check_ctx(c)) return NOVA_B200_INVALID_ARGUMENT;
+  std::ifstream f;
   std::vector<unsigned char> bytes;
-  nova_b200_status st = read_file(c, path, bytes);
+  size_t size = 0;
+  nova_b200_status st = read_head(c, path, f, kHeadBytes, bytes, size);
   if (st) return st;
+  bool done = false;
+  st = read_rows_on_device(c, f, bytes, size, rgba_host, rgba_device, capacity, &done);
+  if (st || done) return st;
+  if ((st = read_rest(c, path, f, bytes, size))) return st;
   Header hd;
   if ((st = parse_header(c, bytes, hd))) return st;
+  if ((st = check_read(c, hd, rgba_device, capacity))) return st;
   const uint64_t npx = (uint64_t)hd.w * hd.h;
-  if (npx > (1ull << 31)) return fail(c, NOVA_B200_INVALID_ARGUMENT, "HDR image larger than 2^31 pixels%s");
-  if (capacity < npx * 4) return fail(c, NOVA_B200_INVALID_ARGUMENT, "output holds fewer than width * height * 4 floats%s");
-  if (rgba_device && (reinterpret_cast<uintptr_t>(rgba_device) & 15))
-    return fail(c, NOVA_B200_INVALID_ARGUMENT, "rgba_device must be 16-byte aligned%s");
   Layout L;
   if ((st = scan_rows(c, bytes, hd, L))) return st;
   cudaSetDevice(c->device);
@@ -601,7 +934,7 @@ extern "C" nova_b200_status nova_b200_hdr_read(nova_b200_ctx *c, const char *pat
                                                                                                n_planes, d_rgbe);
     const uint64_t threads = (npx + 3) / 4;
     k_rgbe_decode<<<(unsigned)((threads + 255) / 256), 256, 0, c->stream>>>(reinterpret_cast<const uint32_t *>(d_rgbe),
-                                                                              npx, d_out);
+                                                                              npx, d_out, nullptr);
     e = cudaGetLastError();
     cudaEventRecord(c->ev_end, c->stream);
   }
