@@ -56,13 +56,15 @@ __device__ __forceinline__ float blend(float acc, float now, float denom) {
   return old + 0.8f * (now - old);
 }
 
+/* From the end of the film: what k_accumulate left of it in the L2 is the end, and the display image goes past
+ * it (3840 x 2160: 77 -> 71 us a call; 398 MB). */
 __global__ void k_display_blend(const float *partial, const float *accum, float *out, uint64_t n, float denom) {
-  const uint64_t i4 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  const uint64_t i4 = ((uint64_t)(gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (i4 + 4 <= n) {
     const float4 p = *reinterpret_cast<const float4 *>(partial + i4);
     const float4 a = *reinterpret_cast<const float4 *>(accum + i4);
-    *reinterpret_cast<float4 *>(out + i4) =
-        make_float4(blend(a.x, p.x, denom), blend(a.y, p.y, denom), blend(a.z, p.z, denom), blend(a.w, p.w, denom));
+    __stcs(reinterpret_cast<float4 *>(out + i4), make_float4(blend(a.x, p.x, denom), blend(a.y, p.y, denom),
+                                                             blend(a.z, p.z, denom), blend(a.w, p.w, denom)));
   } else {
     for (uint64_t i = i4; i < n; i++) out[i] = blend(accum[i], partial[i], denom);
   }
