@@ -1,7 +1,8 @@
 /* Wavefront path tracer: the reference's PathIntegrator::Li (integrator/Integrator.cpp:60-99) as
  * sm_100a kernels over a path queue in HBM, for one frame or a batch of frames of different scenes.
  *
- *   k_refill   fills free queue slots with camera rays of new paths (Integrator.h:66-85 with the
+ *   k_refill   (first waves of frames that start small; others make their camera rays in k_trace) fills
+ *              free queue slots with camera rays of new paths (Integrator.h:66-85 with the
  *              OptiX raygen's sample index (x * H + y) * spp + s, integrator_optix.cu:43; Sobol
  *              dimensions 0 and 1 jitter NDC)
  *   k_trace    closest hit per queued ray (traverse.cuh); a miss finishes its path with the
@@ -54,10 +55,11 @@ using namespace nb;
 
 constexpr uint32_t kQueueCapDefault = 1u << 23; /* rays per wave unless tuned */
 /* Radiance buffer: all of a call's paths up to kRadianceCapBytes, else chunks of kRadianceChunkBytes.  Nothing
- * reuses a chunked call's radiance, so its chunks need only be long against their drain (0.35 ms each): 2^31
- * paths took 294 ms in chunks of 4 GiB, 297 in 2, 303 in 1, 307 in 0.75 and 315 in 0.5 GiB (307 in chunks of
- * 4 GiB before the waves were made shorter), and 0.75 GiB leaves the rest to the other contexts on the GPU. */
-constexpr size_t kRadianceCapBytes = 4ull << 30, kRadianceChunkBytes = 768ull << 20;
+ * reuses a chunked call's radiance, so its chunks need only be long against their drain (0.35 ms each), and
+ * the rest of the memory is left to the other contexts on the GPU: 2^31 paths take 286 ms in chunks of
+ * 4 GiB, 300 in 768 MiB, 304 in 640, 306 in 544 and 309 in 512 (306 in chunks of 4 GiB before the waves
+ * were made shorter). */
+constexpr size_t kRadianceCapBytes = 4ull << 30, kRadianceChunkBytes = 544ull << 20;
 constexpr unsigned kRRDimBase = 200; /* Russian roulette decisions use Sobol dimension 200 + bounce */
 constexpr int kMaxDepth = 48;        /* 2 + 4 (depth + 1) Sobol dimensions must stay below 200 */
 
@@ -240,14 +242,14 @@ __device__ __forceinline__ CameraPath camera_path(const JS &js, uint32_t g) {
   return c;
 }
 
-/* Camera ray of new path `next + i` into queue slot `n_active + i`. */
+/* Camera ray of new path `next + i` into queue slot `n_active + i`; o4, d4: its queue entries. */
 template <class JS>
 __device__ __forceinline__ void refill_one(const Queue &q, uint32_t next, uint32_t n_active, float4 *L, const JS &js,
-                                           uint32_t i) {
+                                           uint32_t i, float4 &o4, float4 &d4) {
   const CameraPath c = camera_path(js, next + i);
   const uint32_t slot = n_active + i;
-  q.o[slot] = make_float4(c.o.x, c.o.y, c.o.z, __uint_as_float(c.rslot));
-  q.d[slot] = make_float4(c.d.x, c.d.y, c.d.z, __uint_as_float(c.job << 8));
+  q.o[slot] = o4 = make_float4(c.o.x, c.o.y, c.o.z, __uint_as_float(c.rslot));
+  q.d[slot] = d4 = make_float4(c.d.x, c.d.y, c.d.z, __uint_as_float(c.job << 8));
   q.beta[slot] = make_float4(1.f, 1.f, 1.f, __uint_as_float(c.index));
   if (js.at(c.job).sc.has_emissive) L[c.rslot] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
@@ -270,9 +272,13 @@ __global__ void __launch_bounds__(256) k_refill(Queue q, WaveCounters *wcp, uint
                                                 uint32_t cap, float4 *L, const __grid_constant__ JS js) {
   const WaveState ws = first_state(wcp, wave, total, cap);
   const uint32_t n_new = min(cap - ws.n_active, total - ws.next);
+  float4 o, d;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += gridDim.x * blockDim.x)
-    refill_one(q, ws.next, ws.n_active, L, js, i);
+    refill_one(q, ws.next, ws.n_active, L, js, i, o, d);
 }
+
+/* What k_refill does to the counters before a first wave that starts its own paths. */
+__global__ void k_start(WaveCounters *wcp, uint32_t total, uint32_t cap) { first_state(wcp, 0, total, cap); }
 
 /* Non-finite radiance becomes 0 (DENAN), counted in *nonfinite (rare: a plain atomic). */
 __device__ __forceinline__ float4 finite_or_zero(V3 L, float alpha, unsigned *nonfinite) {
@@ -350,8 +356,13 @@ constexpr int kTraceBlocks = WIDTH == 1 ? 9 : 10;
  * equal (shading -0.6 %, the third append +0.4 % in k_trace). */
 
 /* The closest-hit pass for one warp's lanes (ray i of n queued; the warp's lanes call together: the
- * hit append is a warp ballot). */
-template <int WIDTH, class JS, bool ADJ, bool COUNT, bool P>
+ * hit append is a warp ballot).
+ *
+ * FRESH, for a wave that starts paths: the lanes past the waiting rays make their camera rays themselves, and
+ * the queue entries they write are for k_shade.  A k_refill before the pass wrote the same entries for it
+ * to read again: 33 M paths at 1920 x 1080 take 8.01 ms so against 8.14, 90 M paths of 8 frames 35.2 against
+ * 35.4.  Camera rays made a second time in k_shade instead of kept in the queue: 8.17 and 35.9. */
+template <int WIDTH, class JS, bool ADJ, bool COUNT, bool P, bool FRESH = false>
 __device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, WaveState &ws, float4 *hits,
                                            uint2 *hit_slot, float4 *L, const JS &js, uint32_t i, uint32_t n) {
   {
@@ -359,7 +370,11 @@ __device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, Wa
     TraceResult r{-1, 0.f, 0.f, 0.f, 0u};
     uint64_t nv = 0, tt = 0;
     if (i < n) {
-      const float4 o = ldq<P>(&q.o[i]), d = ldq<P>(&q.d[i]);
+      float4 o, d;
+      if (FRESH && i >= ws.n_active)
+        refill_one(q, ws.next, ws.n_active, L, js, i - ws.n_active, o, d);
+      else
+        o = ldq<P>(&q.o[i]), d = ldq<P>(&q.d[i]);
       const DevScene &sc = js.at(__float_as_uint(d.w) >> 8).sc;
       if constexpr (P)
         r = walk<WIDTH>(sc, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z});
@@ -405,7 +420,7 @@ __device__ __forceinline__ void trace_warp(const Queue &q, WaveCounters *wcp, Wa
   }
 }
 
-template <int WIDTH, class JS, bool ADJ = false, bool COUNT = false>
+template <int WIDTH, class JS, bool ADJ = false, bool COUNT = false, bool FRESH = false>
 __global__ void __launch_bounds__(128, kTraceBlocks<WIDTH>)
     k_trace(Queue q, WaveCounters *wcp, uint32_t wave, float4 *hits, uint2 *hit_slot, float4 *L,
             const __grid_constant__ JS js) {
@@ -414,7 +429,7 @@ __global__ void __launch_bounds__(128, kTraceBlocks<WIDTH>)
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) advance_wave(wcp, wave);
   if ((i & ~31u) >= n) return; /* whole warps leave together (the append is a warp ballot) */
-  trace_warp<WIDTH, JS, ADJ, COUNT, false>(q, wcp, ws, hits, hit_slot, L, js, i, n);
+  trace_warp<WIDTH, JS, ADJ, COUNT, false, FRESH>(q, wcp, ws, hits, hit_slot, L, js, i, n);
 }
 
 /* Persistent variant of k_trace (binary BVH): a fixed grid of warps hands out the queued rays with
@@ -946,7 +961,8 @@ __global__ void __launch_bounds__(128, NB_PERSIST_MIN_BLOCKS) k_persist(Queue qa
     const uint32_t total = __ldcg(&wcp->total), cap = __ldcg(&wcp->cap);
     if (__ldcg(&wcp->done)) return;
     const uint32_t n_new = min(cap - n_active, total - next), n = n_active + n_new;
-    for (uint32_t i = tid; i < n_new; i += nthreads) refill_one(in, next, n_active, L, js, i);
+    float4 o, d;
+    for (uint32_t i = tid; i < n_new; i += nthreads) refill_one(in, next, n_active, L, js, i, o, d);
     if (!grid_barrier(sync, limit_ns)) return;
     const unsigned long long t0 = leader ? global_ns() : 0ull;
     for (;;) {
@@ -1197,7 +1213,13 @@ cudaError_t enqueue_wave(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, 
   if constexpr (ADJ) ain = slot ? adj->qb : adj->qa, aout = slot ? adj->qa : adj->qb;
   auto blocks = [](uint32_t n, uint32_t block) { return std::max(1u, (n + block - 1) / block); };
   cudaEvent_t *ev = c->ev_wave + 3 * slot;
-  if (p.fresh) {
+  const bool fused = !ADJ && p.fresh && !p.finish && ls.trace_mode == 0;
+  if (fused) {
+    if (p.wave == 0) { /* the trace pass makes the camera rays; something has to start its counters */
+      k_start<<<1, 1, 0, c->stream>>>(b.wc, p.total, p.cap);
+      kernels++;
+    }
+  } else if (p.fresh) {
     const unsigned g = blocks(p.fresh, 256);
     if constexpr (ADJ)
       k_refill_adj<JS><<<g, 256, 0, c->stream>>>(in, ain, b.wc, p.wave, p.total, p.cap, c->d_radiance, adj->d_image, js);
@@ -1231,6 +1253,9 @@ cudaError_t enqueue_wave(nova_b200_ctx *c, const JS &js, const LaunchShape &ls, 
             in, b.wc, p.wave, b.hits, b.hit_slot, c->d_radiance, js);
       } else if (ls.trace_mode == 2) {
         k_trace<WIDTH, JS, false, true>
+            <<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, p.wave, b.hits, b.hit_slot, c->d_radiance, js);
+      } else if (fused) {
+        k_trace<WIDTH, JS, false, false, true>
             <<<g_trace, ls.trace_block, 0, c->stream>>>(in, b.wc, p.wave, b.hits, b.hit_slot, c->d_radiance, js);
       } else {
         k_trace<WIDTH, JS>
