@@ -35,7 +35,8 @@ template <int KIND>
 constexpr int kAovBlocks = KIND == NOVA_B200_AOV_DEPTH ? 10 : KIND == NOVA_B200_AOV_NORMAL ? 8 : 6;
 
 /* One kernel per BVH width and image: with every walk and all three images in one kernel it took 86
- * registers, 5 resident blocks for a walk that waits on its node loads. */
+ * registers, 5 resident blocks for a walk that waits on its node loads: 163 k triangles at 961 x 541, a
+ * depth image took 101 us a call so and 80 this way, normals 105 and 85. */
 template <int WIDTH, int KIND>
 __global__ void __launch_bounds__(128, kAovBlocks<KIND>) k_aov(DevScene sc, const AovParams p, float4 *out) {
   /* a warp takes a tile of 8 x 4 pixels and a block 16 x 8: neighbouring rays walk alike */

@@ -115,6 +115,17 @@ struct UploadPlan {
   }
 };
 
+nova_b200_status ensure_pinned_stage(nova_b200_ctx *c, size_t bytes) {
+  if (c->h_stage_bytes >= bytes) return NOVA_B200_SUCCESS;
+  if (c->h_stage) cudaFreeHost(c->h_stage);
+  c->h_stage = nullptr;
+  c->h_stage_bytes = 0;
+  const size_t want = std::max<size_t>(bytes, 1 << 20);
+  NB_CUDA(c, cudaMallocHost(&c->h_stage, want), "cudaMallocHost(upload staging)");
+  c->h_stage_bytes = want;
+  return NOVA_B200_SUCCESS;
+}
+
 /* One small piece read by the device straight from the caller's pinned host memory. */
 struct GatherPiece {
   const char *src; /* device-accessible address of pinned host memory */
@@ -164,7 +175,7 @@ nova_b200_status copy_pieces(nova_b200_ctx *c, const UploadPlan &plan, char *are
     }
   }
   const size_t table = gather.size() * sizeof(GatherPiece);
-  nova_b200_status st = nb_ensure_stage(c, small + table + 256);
+  nova_b200_status st = ensure_pinned_stage(c, small + table + 256);
   if (st != NOVA_B200_SUCCESS) return st;
   if (!gather.empty()) {
     /* the table goes at the end of the staging buffer, read by the kernel over the bus as well */
@@ -699,17 +710,6 @@ nova_b200_status for_each_context(nova_b200_ctx *const *ctxs, uint32_t n, Op op)
 }
 
 }  // namespace
-
-nova_b200_status nb_ensure_stage(nova_b200_ctx *c, size_t bytes) {
-  if (c->h_stage_bytes >= bytes) return NOVA_B200_SUCCESS;
-  if (c->h_stage) cudaFreeHost(c->h_stage);
-  c->h_stage = nullptr;
-  c->h_stage_bytes = 0;
-  const size_t want = std::max<size_t>(bytes, 1 << 20);
-  NB_CUDA(c, cudaMallocHost(&c->h_stage, want), "cudaMallocHost(upload staging)");
-  c->h_stage_bytes = want;
-  return NOVA_B200_SUCCESS;
-}
 
 extern "C" {
 

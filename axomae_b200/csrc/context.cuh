@@ -23,7 +23,7 @@ struct nova_b200_ctx {
 
   /* scene */
   void *d_arena = nullptr;      /* every scene buffer (textures, meshes, tables) in one pool allocation */
-  void *h_stage = nullptr;      /* pinned staging: small pieces of an upload, pieces of a file */
+  void *h_stage = nullptr;      /* pinned upload staging for small pieces */
   size_t h_stage_bytes = 0;
   nb::DevScene scene{};
   std::vector<nb::DevInstance> h_instances;
@@ -106,9 +106,6 @@ inline nova_b200_status cuda_fail(nova_b200_ctx *c, cudaError_t e, const char *w
     cudaError_t nb_e_ = (call);                                         \
     if (nb_e_ != cudaSuccess) return nbctx::cuda_fail((ctx), nb_e_, where); \
   } while (0)
-
-/* Grows the context's pinned staging (h_stage) to `bytes`, 1 MB at least; nothing may be reading it. */
-nova_b200_status nb_ensure_stage(nova_b200_ctx *c, size_t bytes);
 
 /* Defined in integrator.cu / bake.cu, called by the C-ABI entry points in context.cu. */
 nova_b200_status nb_render(nova_b200_ctx *c, const nova_b200_frame *f, float *film_host, float *film_device,

@@ -24,6 +24,7 @@
 #include <climits>
 #include <cstring>
 #include <fstream>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -709,16 +710,17 @@ nova_b200_status check_read(nova_b200_ctx *c, const Header &hd, const float *rgb
   return NOVA_B200_SUCCESS;
 }
 
-/* hdr_read of a run-length file of more than kDeviceBytes or kDevicePixels: the bytes go through the context's pinned staging to
- * the device as they are read, and the device finds, checks and expands the rows.  *done stays false when
- * this is no such file, or one whose rows it could not chain: nothing has been written then, and the
- * caller reads the file the other way, which also says what is wrong with it.
+/* hdr_read of a run-length file of more than kDeviceBytes or kDevicePixels: the bytes go to the device in pieces
+ * as they are read, and the device finds, checks and expands the rows.  *done stays false when this is no
+ * such file, or one whose rows it could not chain: nothing has been written then, and the caller reads
+ * the file the other way, which also says what is wrong with it.
  *
  * The other way's walk of the packets on the host costs 2.5 ns a packet, this one five short kernels and their
- * gaps.  Random values (few packets a byte): 78 KB 75 us the other way and 102 this way, 256 KB 107 and 116,
- * 513 KB 153 and 126, 2 MB 550 and 271, 32 MB 8.4 and 3.0 ms; one colour (66 values a byte, so the pixels
- * tell): 0.5 Mpixel 81 and 92, 2 Mpixel 160 and 120, 8 Mpixel 450 and 240. */
-constexpr size_t kHeadBytes = 1 << 16, kFilePiece = 1 << 18, kRowSmem = 200 << 10;
+ * gaps.  Random values (few packets a byte): 128 KB 83 us the other way and 101 this way, 320 KB 121 and 120,
+ * 513 KB 155 and 136, 2 MB 555 and 317, 32 MB 8.4 and 3.1 ms; one colour (66 values a byte, so the pixels
+ * tell): 0.5 Mpixel 81 and 92, 2 Mpixel 160 and 120, 8 Mpixel 450 and 241.  Pieces of 64 to 256 KB are
+ * slower and uneven (2 MB: 330 to 370 us), pinned ones 290, but pinning 1 MB costs a new context 1.3 ms. */
+constexpr size_t kHeadBytes = 1 << 16, kFilePiece = 1 << 20, kRowSmem = 200 << 10;
 constexpr size_t kDeviceBytes = 5 << 16, kDevicePixels = 1 << 20;
 
 nova_b200_status read_rows_on_device(nova_b200_ctx *c, std::ifstream &f, const std::vector<unsigned char> &head,
@@ -737,7 +739,6 @@ nova_b200_status read_rows_on_device(nova_b200_ctx *c, std::ifstream &f, const s
   nova_b200_status st = check_read(c, hd, rgba_device, capacity);
   if (st) return st;
   cudaSetDevice(c->device);
-  if ((st = nb_ensure_stage(c, 4 * kFilePiece))) return st;
   const uint64_t npx = (uint64_t)hd.w * hd.h;
   const uint32_t h = (uint32_t)hd.h;
   const uint64_t tiles = (n + kFindTile - 1) / kFindTile, per = (tiles + kFindBlocks - 1) / kFindBlocks;
@@ -762,13 +763,11 @@ nova_b200_status read_rows_on_device(nova_b200_ctx *c, std::ifstream &f, const s
   if (e == cudaSuccess) e = cudaMemsetAsync(d_ok, 0xff, sizeof(uint32_t) * (1 + (size_t)most), c->stream);
   bool read = true;
   f.seekg((std::streamoff)hd.data);
-  const size_t slots = c->h_stage_bytes / kFilePiece;
-  for (uint64_t off = 0, k = 0; e == cudaSuccess && read && off < n; off += kFilePiece, k++) {
-    if (k % slots == 0) e = cudaStreamSynchronize(c->stream); /* the copies out of the staging are done */
-    char *piece = static_cast<char *>(c->h_stage) + (k % slots) * kFilePiece;
+  const std::unique_ptr<char[]> piece(new char[(size_t)std::min<uint64_t>(n, kFilePiece)]);
+  for (uint64_t off = 0; e == cudaSuccess && read && off < n; off += kFilePiece) {
     const size_t bytes = (size_t)std::min<uint64_t>(kFilePiece, n - off);
-    read = (bool)f.read(piece, (std::streamsize)bytes);
-    if (e == cudaSuccess && read) e = cudaMemcpyAsync(d_body + off, piece, bytes, cudaMemcpyHostToDevice, c->stream);
+    read = (bool)f.read(piece.get(), (std::streamsize)bytes);
+    if (read) e = cudaMemcpyAsync(d_body + off, piece.get(), bytes, cudaMemcpyHostToDevice, c->stream);
   }
   uint32_t ok = 0;
   if (e == cudaSuccess && read) {
