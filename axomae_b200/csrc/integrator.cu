@@ -45,6 +45,7 @@
 #include <thread>
 #include <vector>
 
+#include "caller_memory.cuh"
 #include "context.cuh"
 #include "shading.cuh"
 #include "traverse.cuh"
@@ -1586,13 +1587,15 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
       if (s) cudaStreamSynchronize(s);
     }
   } copies_done{nc > 1 ? x->copy_stream : nullptr};
-  /* where a frame's last resolve writes its film: the caller's device film itself when it is aligned, which
+  /* where a frame's last resolve writes its film: the caller's device film itself where it may, which
    * saves a copy of it; earlier chunks of the frame write the context's, so that a render that fails
    * leaves the caller's alone */
-  auto film_target = [&](size_t j) {
-    float *f = films_device ? films_device[j] : nullptr;
-    return f && !(reinterpret_cast<uintptr_t>(f) & 15u) ? f : ctxs[j]->d_film_out;
-  };
+  std::vector<Span> spans(nj, Span{0, 0});
+  for (size_t j = 0; films_device && j < nj; j++)
+    spans[j] = Span{reinterpret_cast<uintptr_t>(films_device[j]),
+                    (size_t)frames[j]->width * frames[j]->height * 4 * sizeof(float)};
+  const std::vector<char> direct = direct_films(spans);
+  auto film_target = [&](size_t j) { return direct[j] ? films_device[j] : ctxs[j]->d_film_out; };
   auto copy_film = [&](size_t j, cudaStream_t stream) -> nova_b200_status {
     const size_t bytes = (size_t)frames[j]->width * frames[j]->height * 4 * sizeof(float);
     const float *film = film_target(j);
