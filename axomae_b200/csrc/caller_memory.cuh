@@ -2,6 +2,8 @@
  * plain values in and out. */
 #pragma once
 
+#include <cuda_runtime_api.h>
+
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
@@ -10,9 +12,16 @@
 
 namespace nb {
 
+/* True for memory of `device` itself.  A copy also takes another GPU's memory, without peer access, and host
+ * memory; a kernel's load or store there would be an illegal address and cost the caller its context. */
+inline bool on_device(const cudaPointerAttributes &a, int device) {
+  return a.type == cudaMemoryTypeDevice && a.device == device;
+}
+
 struct Span {
   uintptr_t begin;
   size_t bytes;
+  bool here; /* on_device of the GPU that does the work */
   uintptr_t end() const { return begin + bytes; }
 };
 
@@ -21,7 +30,7 @@ struct Span {
  * frames: a program that takes every frame's film to the host may pass one device buffer for all. */
 inline std::vector<char> direct_films(const std::vector<Span> &films) {
   std::vector<char> direct(films.size());
-  for (size_t j = 0; j < films.size(); j++) direct[j] = films[j].begin != 0 && (films[j].begin & 15u) == 0;
+  for (size_t j = 0; j < films.size(); j++) direct[j] = films[j].here && films[j].begin != 0 && (films[j].begin & 15u) == 0;
   std::vector<size_t> at(films.size()); /* by address; `last` reaches furthest of those before */
   std::iota(at.begin(), at.end(), size_t{0});
   std::sort(at.begin(), at.end(), [&](size_t a, size_t b) { return films[a].begin < films[b].begin; });

@@ -1590,10 +1590,13 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
   /* where a frame's last resolve writes its film: the caller's device film itself where it may, which
    * saves a copy of it; earlier chunks of the frame write the context's, so that a render that fails
    * leaves the caller's alone */
-  std::vector<Span> spans(nj, Span{0, 0});
-  for (size_t j = 0; films_device && j < nj; j++)
+  std::vector<Span> spans(nj, Span{0, 0, false});
+  for (size_t j = 0; films_device && j < nj; j++) {
+    cudaPointerAttributes at{};
+    if (films_device[j] && cudaPointerGetAttributes(&at, films_device[j]) != cudaSuccess) cudaGetLastError();
     spans[j] = Span{reinterpret_cast<uintptr_t>(films_device[j]),
-                    (size_t)frames[j]->width * frames[j]->height * 4 * sizeof(float)};
+                    (size_t)frames[j]->width * frames[j]->height * 4 * sizeof(float), on_device(at, x->device)};
+  }
   const std::vector<char> direct = direct_films(spans);
   auto film_target = [&](size_t j) { return direct[j] ? films_device[j] : ctxs[j]->d_film_out; };
   auto copy_film = [&](size_t j, cudaStream_t stream) -> nova_b200_status {
