@@ -15,6 +15,7 @@
  * trigonometry in float.  This file is compiled with the default multiply-add contraction, like the
  * reference's CUDA sources (its CMake flags only add --expt-relaxed-constexpr -std=c++17).
  */
+#include "caller_memory.cuh"
 #include "context.cuh"
 
 namespace {
@@ -148,7 +149,7 @@ nova_b200_status nb_bake_texunit(nova_b200_ctx *c, const float *src, int32_t sw,
   if (sw > max_w || sh > max_h) return fail(c, NOVA_B200_INVALID_ARGUMENT, "source map larger than a 2D texture%s");
   cudaSetDevice(c->device);
   /* The texture reads linear memory where its limits allow: the caller's own map when its base and rows
-   * are aligned, else an aligned copy from the pool.  An array of its own per call took cudaMallocArray
+   * are aligned and the bake does not write over it, else an aligned copy from the pool.  An array of its own per call took cudaMallocArray
    * and cudaFreeArray, 0.4 of the call's 0.55 ms at 1024 x 512 (and now and then tens of ms); the texture
    * unit filters both alike.  Larger maps still get the array. */
   const size_t texels = (size_t)sw * sh;
@@ -162,8 +163,10 @@ nova_b200_status nb_bake_texunit(nova_b200_ctx *c, const float *src, int32_t sw,
   const size_t row = (size_t)sw * sizeof(float4);
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, src) != cudaSuccess) cudaGetLastError();
-  const bool direct = ch == 4 && at.type == cudaMemoryTypeDevice &&
-                      aligned(reinterpret_cast<uintptr_t>(src), tex_align) && aligned(row, pitch_align);
+  const nb::Span map{reinterpret_cast<uintptr_t>(src), row * sh, at.type == cudaMemoryTypeDevice};
+  const nb::Span target{reinterpret_cast<uintptr_t>(out), sizeof(float4) * (size_t)ow * oh, true};
+  const bool direct = ch == 4 && map.here && !nb::overlap(map, target) && aligned(map.begin, tex_align) &&
+                      aligned(row, pitch_align);
   const size_t pitch = direct ? row : (row + tex_align - 1) / tex_align * tex_align;
   const bool linear = sw <= lin_w && sh <= lin_h && pitch <= (size_t)lin_pitch;
   const cudaChannelFormatDesc fmt = cudaCreateChannelDesc(32, 32, 32, 32, cudaChannelFormatKindFloat);

@@ -25,6 +25,8 @@ struct Span {
   uintptr_t end() const { return begin + bytes; }
 };
 
+inline bool overlap(const Span &a, const Span &b) { return a.begin < b.end() && b.begin < a.end(); }
+
 /* Per film of a call (begin 0: none): 1 where the kernel that finishes it may store to it.  Its stores are
  * 16 bytes wide.  Films that share memory keep a buffer each until they are copied out, in the order of the
  * frames: a program that takes every frame's film to the host may pass one device buffer for all. */

@@ -26,6 +26,12 @@ int main() {
   check(!nb::on_device(at(cudaMemoryTypeUnregistered, -2), 0), "pageable host memory");
   check(!nb::on_device(cudaPointerAttributes{}, 0), "a pointer without attributes");
 
+  check(nb::overlap({4096, 64, true}, {4096, 64, true}) && nb::overlap({4096, 64, true}, {4159, 64, true}) &&
+            nb::overlap({4159, 64, true}, {4096, 64, true}) && nb::overlap({4096, 64, true}, {4100, 4, true}),
+        "spans that overlap");
+  check(!nb::overlap({4096, 64, true}, {4160, 64, true}) && !nb::overlap({4160, 64, true}, {4096, 64, true}),
+        "spans end to end");
+
   check(direct({}) == Want{}, "no films");
   check(direct({{4096, 64, true}}) == Want{1}, "one film");
   check(direct({{0, 64, false}, {0, 64, false}}) == (Want{0, 0}), "no device films");
