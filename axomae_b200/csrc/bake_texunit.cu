@@ -109,11 +109,11 @@ __global__ void __launch_bounds__(128) k_bake_texunit(float *out, cudaTextureObj
   o[3] = 1.f;
 }
 
-/* RGB(A) source -> RGBA rows of `pitch` bytes with alpha 1, as TextureProcessing.cpp:24-32 prepares it. */
-__global__ void k_to_rgba(const float *src, int w, size_t n, int ch, char *dst, size_t pitch) {
+/* RGB source -> RGBA rows of `pitch` bytes with alpha 1, as TextureProcessing.cpp:24-32 prepares it. */
+__global__ void k_to_rgba(const float *src, int w, size_t n, char *dst, size_t pitch) {
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
     const size_t y = k / (size_t)w, x = k - y * (size_t)w;
-    reinterpret_cast<float4 *>(dst + y * pitch)[x] = make_float4(src[k * ch], src[k * ch + 1], src[k * ch + 2], 1.f);
+    reinterpret_cast<float4 *>(dst + y * pitch)[x] = make_float4(src[3 * k], src[3 * k + 1], src[3 * k + 2], 1.f);
   }
 }
 
@@ -148,10 +148,11 @@ nova_b200_status nb_bake_texunit(nova_b200_ctx *c, const float *src, int32_t sw,
   cudaDeviceGetAttribute(&max_h, cudaDevAttrMaxTexture2DHeight, c->device);
   if (sw > max_w || sh > max_h) return fail(c, NOVA_B200_INVALID_ARGUMENT, "source map larger than a 2D texture%s");
   cudaSetDevice(c->device);
-  /* The texture reads linear memory where its limits allow: the caller's own map when its base and rows
-   * are aligned and the bake does not write over it, else an aligned copy from the pool.  An array of its own per call took cudaMallocArray
-   * and cudaFreeArray, 0.4 of the call's 0.55 ms at 1024 x 512 (and now and then tens of ms); the texture
-   * unit filters both alike.  Larger maps still get the array. */
+  /* The texture reads linear memory where its limits allow: the caller's own map when it lies on this GPU,
+   * its base and rows are aligned and the bake does not write over it, else an aligned copy from the pool.
+   * RGBA maps are copied by the copy engine's rules, which take another GPU's memory too.  An array of its
+   * own per call took cudaMallocArray and cudaFreeArray, 0.4 of the call's 0.55 ms at 1024 x 512 (and now
+   * and then tens of ms); the texture unit filters both alike.  Larger maps still get the array. */
   const size_t texels = (size_t)sw * sh;
   int lin_w = 0, lin_h = 0, lin_pitch = 0, tex_align = 512, pitch_align = 32;
   cudaDeviceGetAttribute(&lin_w, cudaDevAttrMaxTexture2DLinearWidth, c->device);
@@ -163,7 +164,7 @@ nova_b200_status nb_bake_texunit(nova_b200_ctx *c, const float *src, int32_t sw,
   const size_t row = (size_t)sw * sizeof(float4);
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, src) != cudaSuccess) cudaGetLastError();
-  const nb::Span map{reinterpret_cast<uintptr_t>(src), row * sh, at.type == cudaMemoryTypeDevice};
+  const nb::Span map{reinterpret_cast<uintptr_t>(src), row * sh, nb::on_device(at, c->device)};
   const nb::Span target{reinterpret_cast<uintptr_t>(out), sizeof(float4) * (size_t)ow * oh, true};
   const bool direct = ch == 4 && map.here && !nb::overlap(map, target) && aligned(map.begin, tex_align) &&
                       aligned(row, pitch_align);
@@ -181,7 +182,10 @@ nova_b200_status nb_bake_texunit(nova_b200_ctx *c, const float *src, int32_t sw,
     rgba = base;
     if (e == cudaSuccess) {
       base += (tex_align - reinterpret_cast<uintptr_t>(base) % tex_align) % tex_align;
-      k_to_rgba<<<592, 256, 0, c->stream>>>(src, sw, texels, ch, base, linear ? pitch : row);
+      if (ch == 4)
+        e = cudaMemcpy2DAsync(base, pitch, src, row, row, (size_t)sh, cudaMemcpyDeviceToDevice, c->stream);
+      else
+        k_to_rgba<<<592, 256, 0, c->stream>>>(src, sw, texels, base, linear ? pitch : row);
       src = reinterpret_cast<const float *>(base);
     }
   }

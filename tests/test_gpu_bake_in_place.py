@@ -26,3 +26,21 @@ def test_texunit_bake_over_its_map(w, h, ow, oh, shift, ch):
         c.close()
     assert torch.isfinite(apart).all() and (apart.view(-1, 4)[:, :3] > 0).all()
     assert torch.equal(apart, memory[shift:n])
+
+
+def test_texunit_bake_of_a_pinned_host_map():
+    """Memory that is not the GPU's own is copied: the same bits as the map in device memory."""
+    import torch
+    from axomae_b200 import native
+    w, h, ow, oh = 128, 64, 64, 32
+    src = torch.from_numpy(np.random.default_rng(3).lognormal(0, 1, (h, w, 4)).astype(np.float32))
+    maps = [src.cuda(), src.pin_memory()]
+    films = [torch.zeros((oh, ow, 4), device="cuda") for _ in maps]
+    torch.cuda.synchronize()
+    c = native.Context(0)
+    try:
+        for m, f in zip(maps, films):
+            c.bake_irradiance_texunit(m.data_ptr(), w, h, 4, ow, oh, 33, f.data_ptr())
+    finally:
+        c.close()
+    assert (films[0][..., :3] > 0).all() and torch.equal(films[0], films[1])
