@@ -1016,9 +1016,15 @@ __global__ void k_resolve(const float4 *L, uint32_t NP, uint32_t count, float4 *
   reinterpret_cast<float4 *>(out)[(size_t)row * W + x] = make_float4(a.x / denom, a.y / denom, a.z / denom, a.w / denom);
 }
 
+/* Resident blocks of 128 threads per SM of the intersector by itself: as in a wave, but for the 8-wide walk,
+ * whose spills at 10 blocks cost more here (1 M incoherent rays on 65 k triangles: 297 us at 10, 294 at 9,
+ * 265 at 8, 268 at 7; 274 with the three walks in one kernel). */
+template <int WIDTH>
+constexpr int kTraceApiBlocks = WIDTH == 8 ? 8 : kTraceBlocks<WIDTH>;
+
 /* One kernel per BVH width: with the three walks in one kernel the registers were the largest walk's. */
 template <int WIDTH>
-__global__ void __launch_bounds__(128, kTraceBlocks<WIDTH>)
+__global__ void __launch_bounds__(128, kTraceApiBlocks<WIDTH>)
     k_trace_api(DevScene sc, uint64_t n, const float *o, const float *d, int32_t *prim, float *t, float *u, float *v) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
