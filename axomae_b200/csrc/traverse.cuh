@@ -519,9 +519,4 @@ NB_D TraceResult walk(const DevScene &sc, V3 o, V3 d) {
   return walk_tables<WIDTH>(WalkTables{sc.nodes, sc.tris, sc.instances, sc.inst_rec}, o, d);
 }
 
-/* The same on the scene's own width. */
-NB_D TraceResult walk_any(const DevScene &sc, V3 o, V3 d) {
-  return sc.width == 8 ? walk<8>(sc, o, d) : sc.width == 1 ? walk<1>(sc, o, d) : walk<2>(sc, o, d);
-}
-
 }  // namespace nb
