@@ -30,15 +30,16 @@ struct AovParams {
   float inv_P[16], inv_V[16];
 };
 
-/* Resident blocks of 128 threads per SM: the depth image is a walk alone, the others add shading. */
-template <int KIND>
-constexpr int kAovBlocks = KIND == NOVA_B200_AOV_DEPTH ? 10 : KIND == NOVA_B200_AOV_NORMAL ? 8 : 6;
+/* Resident blocks of 128 threads per SM: the depth image is a walk alone (the 8-wide one spills at 10), the
+ * others add shading. */
+template <int WIDTH, int KIND>
+constexpr int kAovBlocks = KIND == NOVA_B200_AOV_DEPTH ? (WIDTH == 8 ? 8 : 10) : KIND == NOVA_B200_AOV_NORMAL ? 8 : 6;
 
 /* One kernel per BVH width and image: with every walk and all three images in one kernel it took 86
  * registers, 5 resident blocks for a walk that waits on its node loads: 163 k triangles at 961 x 541, a
  * depth image took 101 us a call so and 80 this way, normals 105 and 85. */
 template <int WIDTH, int KIND>
-__global__ void __launch_bounds__(128, kAovBlocks<KIND>) k_aov(DevScene sc, const AovParams p, float4 *out) {
+__global__ void __launch_bounds__(128, kAovBlocks<WIDTH, KIND>) k_aov(DevScene sc, const AovParams p, float4 *out) {
   /* a warp takes a tile of 8 x 4 pixels and a block 16 x 8: neighbouring rays walk alike */
   int x, y;
   if (p.linear) {
