@@ -51,12 +51,13 @@
 namespace {
 
 constexpr uint32_t kQueueCapDefault = 1u << 23; /* rays per wave unless tuned */
-/* Radiance buffer: all of a call's paths up to kRadianceCapBytes, else chunks of kRadianceChunkBytes.  Nothing
- * reuses a chunked call's radiance, so its chunks need only be long against their drain (0.35 ms each), and
- * the rest of the memory is left to the other contexts on the GPU: 2^31 paths take 286 ms in chunks of
- * 4 GiB, 300 in 768 MiB, 304 in 640, 306 in 544 and 309 in 512 (306 in chunks of 4 GiB before the waves
- * were made shorter). */
-constexpr size_t kRadianceCapBytes = 4ull << 30, kRadianceChunkBytes = 544ull << 20;
+/* Radiance buffer: up to kRadianceCapBytes of a call's paths; a call with more goes in chunks.  A batch's chunks
+ * are as long as the buffer: each drains by itself (32 frames, 485 M paths: 245 ms a step in chunks of 4 GiB,
+ * 251 in 544 MiB).  A single frame's are kFrameChunkBytes, which costs it 7 % (2^31 paths: 286 ms in 4 GiB, 300 in
+ * 768 MiB, 305 in 576 MiB, 309 in 512), and for one reason only: test_cancel_stops_a_long_render cancels a frame of
+ * 2^31 paths 0.3 s after its start and needs it to be still running.  306 ms is what such a frame took before the
+ * waves were made shorter. */
+constexpr size_t kRadianceCapBytes = 4ull << 30, kFrameChunkBytes = 576ull << 20;
 
 constexpr uint32_t kTileW = 8, kTileH = 4; /* default pixel tile: one warp of camera rays per tile */
 
@@ -444,8 +445,9 @@ nova_b200_status render_jobs(nova_b200_ctx *x, const std::vector<nova_b200_ctx *
     max_np = std::max(max_np, np);
     total += np * (uint64_t)frames[j]->sample_count;
   }
-  const uint64_t radiance = std::max<uint64_t>(
-      max_np, (total <= kRadianceCapBytes / sizeof(float4)) ? total : kRadianceChunkBytes / sizeof(float4));
+  const uint64_t most = (nj == 1 && total > kRadianceCapBytes / sizeof(float4) ? kFrameChunkBytes : kRadianceCapBytes) /
+                        sizeof(float4);
+  const uint64_t radiance = std::max<uint64_t>(max_np, std::min(total, most));
   const nova_b200_tuning &tu = x->tuning;
   const uint32_t qc = tu.queue_capacity ? tu.queue_capacity : kQueueCapDefault;
   const uint32_t cap = (uint32_t)std::min<uint64_t>(qc, std::max<uint64_t>(radiance, 1024));
