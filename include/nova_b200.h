@@ -112,8 +112,10 @@ typedef struct {
   int32_t bins;          /* SAH bins per axis, 4..32; 0 = default (16) */
   int32_t width;         /* 2: binary BVH (default, fastest measured); 8: compressed 8-wide BVH; 0 = 2 */
   int32_t small_subtree; /* nodes of at most this many triangles are built whole by one thread block
-                            (64..65536, above 256 as 256; 0 = default 256); a build-speed knob, the tree
-                            is the same either way */
+                            (64..65536, above 256 as 256; 0 = default 256); a build-speed knob.  Hits are
+                            the same either way, and the tree's kind; its nodes may differ where no
+                            plane separates triangles of equal box centres: they are halved in the
+                            order they lie in, and above this size with the parent's box */
 } nova_b200_bvh_options;
 
 /* One render call.  Samples [sample_begin, sample_begin + sample_count) of every pixel are traced and
