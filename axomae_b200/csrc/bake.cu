@@ -164,7 +164,7 @@ __device__ __forceinline__ V3 bake_sum(const Src &src, const float *lut, const T
 
 /* G lanes per output texel.  Bound by instruction issue (84 % of the slots, 28 of 32 lanes): about 500 a
  * sample, 91 of them in double precision.  512 x 256 texels x 128 samples of a 2048 x 1024 map, one call:
- * 507 us with four texel loads and five double-precision functions a sample, 281 us with one load and
+ * 507 us with four texel loads and five double-precision functions a sample, 264 us with one load and
  * three (the source read for non-finite texels included).  256 x 128 texels, where one thread per texel
  * fills a tenth of the GPU: 347 us with one lane, 99 with eight. */
 template <int G>
@@ -196,12 +196,15 @@ __global__ void __launch_bounds__(128) k_bake(Src src, const float *lut, const u
   o[2] = irr.z;
 }
 
-/* Lanes per texel: the fewest of 1, 2, 4, 8 that fill the GPU's threads twice over.  Each lane adds all
- * of its group's samples, so more lanes than that cost (6 instructions a sample and lane); 131,072
- * texels take 4: 285 us against 291 with 1. */
+/* Lanes per texel: the fewest of 1, 2, 4, 8 that give every thread the GPU holds a lane.  Each lane adds all of
+ * its group's samples (6 instructions a sample and lane) and makes the texel's frame, so more lanes than that
+ * cost.  128 samples of a 2048 x 1024 map with 1, 2, 4 and 8 lanes: 32,768 texels 176, 109, 93 and 92 us, 65,536
+ * 195, 157, 151 and 155, 131,072 284, 266, 266 and 278 (33 samples 91, 90, 97 and 113), 262,144 499, 482, 492 and
+ * 522, 524,288 927, 915, 943 and 1017.  Where the loads miss the L2 more lanes hide more of them: 131,072 texels of
+ * an 8192 x 4096 map 715 us with 4, 683 with 8. */
 int bake_lanes(uint64_t texels) {
   int g = 1;
-  while (g < 8 && texels * g < 2ull * 148 * 2048) g *= 2;
+  while (g < 8 && texels * g < 148ull * 2048) g *= 2;
   return g;
 }
 

@@ -6,8 +6,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-FILL = 2 * 148 * 2048  # threads that fill the GPU twice over
-SIZES = [(256, 256, 8), (512, 256, 8), (512, 512, 4), (1024, 512, 2), (1024, 1024, 1)]
+FILL = 148 * 2048  # threads that the GPU holds
+SIZES = [(256, 256), (512, 256), (512, 512), (1024, 512), (1024, 1024)]
 
 
 @pytest.fixture(scope="module")
@@ -18,16 +18,17 @@ def ctx():
     c.close()
 
 
-def _lanes(texels):
-    return next(g for g in (1, 2, 4, 8) if g == 8 or texels * g >= FILL)
+def test_sizes_reach_every_lane_count():
+    """The rules: the fewest lanes that fill the GPU once (CPU bake) and twice (texture unit)."""
+    for fill in (FILL, 2 * FILL):
+        assert {next(g for g in (1, 2, 4, 8) if g == 8 or w * h * g >= fill) for w, h in SIZES} == {1, 2, 4, 8}
 
 
-@pytest.mark.parametrize("ow,oh,lanes", SIZES)
+@pytest.mark.parametrize("ow,oh", SIZES)
 @pytest.mark.parametrize("samples", [1, 5])
-def test_bake(ctx, ow, oh, lanes, samples):
+def test_bake(ctx, ow, oh, samples):
     import torch
     import oracle_binding
-    assert _lanes(ow * oh) == lanes
     src = np.random.default_rng(ow + samples).lognormal(0, 1, (21, 43, 4)).astype(np.float32)
     ts, out = torch.from_numpy(src).cuda(), torch.zeros((oh, ow, 4), device="cuda")
     torch.cuda.synchronize()
@@ -36,9 +37,9 @@ def test_bake(ctx, ow, oh, lanes, samples):
     np.testing.assert_allclose(out.cpu().numpy()[..., :3], ref[..., :3], rtol=1e-4, atol=1e-6)
 
 
-@pytest.mark.parametrize("ow,oh,lanes", SIZES)
+@pytest.mark.parametrize("ow,oh", SIZES)
 @pytest.mark.parametrize("samples", [1, 5])
-def test_texunit_bake(ctx, ow, oh, lanes, samples):
+def test_texunit_bake(ctx, ow, oh, samples):
     """A filter weight of the texture unit has 8 fractional bits, and rounding in the trigonometry may move each of
     the two by one step: 2 / 256 of the map's range a sample, so as much of their mean, where one sample
     lost or counted twice is a tenth of the range at least.  At a pole the azimuth is all rounding: one texel in
