@@ -20,7 +20,9 @@ struct BvhBuildResult {
   double ms;
 };
 
-/* Builds a binary BVH over n primitive boxes (lo/hi: world-space, float4 with w unused).
+/* Builds a binary BVH over n primitive boxes (lo/hi: world-space, float4 with w unused; no coordinate -0, which
+ * the build's float minima by integer atomics would take for the least value of all, cutting boxes off at zero:
+ * making it +0 in every atomic took 5 % of a 3 M triangle build, in the boxes nothing).
  * nodes: room for n + 1 nodes (4 float4 each, layout in device_scene.cuh).
  * order: receives, for every leaf slot, the index (into lo/hi) of the primitive stored there.
  * Returns a CUDA error code (cudaSuccess on success). */

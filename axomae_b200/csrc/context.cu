@@ -242,6 +242,12 @@ void free_scene(nova_b200_ctx *c) {
 
 /* ------------------------------------------------------------------ build kernels */
 
+/* One of build_bvh's boxes: no coordinate is -0 (the sum makes it +0). */
+__device__ __forceinline__ void write_box(float4 *lo, float4 *hi, nb::V3 l, nb::V3 h) {
+  *lo = make_float4(l.x + 0.f, l.y + 0.f, l.z + 0.f, 0.f);
+  *hi = make_float4(h.x + 0.f, h.y + 0.f, h.z + 0.f, 0.f);
+}
+
 __global__ void k_prim_boxes(nb::DevScene sc, const uint32_t *valid, uint32_t n, float4 *lo, float4 *hi) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -255,10 +261,11 @@ __global__ void k_prim_boxes(nb::DevScene sc, const uint32_t *valid, uint32_t n,
     const nb::V3 v = nb::vertex_position(m, m.idx[3 * tri + k]);
     w[k] = I.identity ? v : nb::xform_point(I.m, v);
   }
-  lo[i] = make_float4(fminf(w[0].x, fminf(w[1].x, w[2].x)), fminf(w[0].y, fminf(w[1].y, w[2].y)),
-                      fminf(w[0].z, fminf(w[1].z, w[2].z)), 0.f);
-  hi[i] = make_float4(fmaxf(w[0].x, fmaxf(w[1].x, w[2].x)), fmaxf(w[0].y, fmaxf(w[1].y, w[2].y)),
-                      fmaxf(w[0].z, fmaxf(w[1].z, w[2].z)), 0.f);
+  write_box(lo + i, hi + i,
+            nb::V3{fminf(w[0].x, fminf(w[1].x, w[2].x)), fminf(w[0].y, fminf(w[1].y, w[2].y)),
+                   fminf(w[0].z, fminf(w[1].z, w[2].z))},
+            nb::V3{fmaxf(w[0].x, fmaxf(w[1].x, w[2].x)), fmaxf(w[0].y, fmaxf(w[1].y, w[2].y)),
+                   fmaxf(w[0].z, fmaxf(w[1].z, w[2].z))});
 }
 
 /* Triangle records in leaf order: (v0, prim id), (v1 - v0, instance), (v2 - v0, 0), object space. */
@@ -445,10 +452,11 @@ __global__ void k_mesh_boxes(nb::DevMesh m, const uint32_t *ids, uint32_t n, flo
   const uint32_t t = ids[i];
   nb::V3 w[3];
   for (int k = 0; k < 3; k++) w[k] = nb::vertex_position(m, m.idx[3 * (size_t)t + k]);
-  lo[i] = make_float4(fminf(w[0].x, fminf(w[1].x, w[2].x)), fminf(w[0].y, fminf(w[1].y, w[2].y)),
-                      fminf(w[0].z, fminf(w[1].z, w[2].z)), 0.f);
-  hi[i] = make_float4(fmaxf(w[0].x, fmaxf(w[1].x, w[2].x)), fmaxf(w[0].y, fmaxf(w[1].y, w[2].y)),
-                      fmaxf(w[0].z, fmaxf(w[1].z, w[2].z)), 0.f);
+  write_box(lo + i, hi + i,
+            nb::V3{fminf(w[0].x, fminf(w[1].x, w[2].x)), fminf(w[0].y, fminf(w[1].y, w[2].y)),
+                   fminf(w[0].z, fminf(w[1].z, w[2].z))},
+            nb::V3{fmaxf(w[0].x, fmaxf(w[1].x, w[2].x)), fmaxf(w[0].y, fmaxf(w[1].y, w[2].y)),
+                   fmaxf(w[0].z, fmaxf(w[1].z, w[2].z))});
 }
 
 /* Bottom-level triangle records in leaf order: (v0, mesh-local triangle id), (v1 - v0, 0), (v2 - v0, 0). */
@@ -504,8 +512,7 @@ __global__ void k_instance_boxes(const nb::DevInstance *inst, uint32_t n, const 
     wl = nb::V3{fminf(wl.x, w.x), fminf(wl.y, w.y), fminf(wl.z, w.z)};
     wh = nb::V3{fmaxf(wh.x, w.x), fmaxf(wh.y, w.y), fmaxf(wh.z, w.z)};
   }
-  lo[i] = make_float4(wl.x, wl.y, wl.z, 0.f);
-  hi[i] = make_float4(wh.x, wh.y, wh.z, 0.f);
+  write_box(lo + i, hi + i, wl, wh);
 }
 
 /* Top-level leaves (one instance each) name the instance itself instead of its slot in `order`. */
