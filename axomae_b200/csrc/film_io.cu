@@ -669,8 +669,11 @@ nova_b200_status scan_rows(nova_b200_ctx *c, const std::vector<unsigned char> &b
   return NOVA_B200_SUCCESS;
 }
 
-/* Opens a file, unbuffered (it is read in large pieces), and reads the first `limit` bytes of its `size`. */
-nova_b200_status read_head(nova_b200_ctx *c, const char *path, std::ifstream &f, size_t limit,
+/* Opens a file, unbuffered (it is read in large pieces), and reads all of its `size` bytes up to `whole`, else the
+ * first kHeadBytes. */
+constexpr size_t kHeadBytes = 1 << 16;
+
+nova_b200_status read_head(nova_b200_ctx *c, const char *path, std::ifstream &f, size_t whole,
                            std::vector<unsigned char> &bytes, size_t &size) {
   using namespace nbctx;
   if (!path) return fail(c, NOVA_B200_INVALID_ARGUMENT, "path is null%s");
@@ -680,7 +683,7 @@ nova_b200_status read_head(nova_b200_ctx *c, const char *path, std::ifstream &f,
   const std::streamoff end = f.tellg();
   if (end < 0) return fail(c, NOVA_B200_INVALID_ARGUMENT, "cannot read %s", path);
   size = (size_t)end;
-  bytes.resize(std::min(size, limit));
+  bytes.resize(size <= whole ? size : std::min(size, kHeadBytes));
   f.seekg(0);
   if (!bytes.empty() && !f.read(reinterpret_cast<char *>(bytes.data()), (std::streamsize)bytes.size()))
     return fail(c, NOVA_B200_INVALID_ARGUMENT, "cannot read %s", path);
@@ -720,16 +723,15 @@ nova_b200_status check_read(nova_b200_ctx *c, const Header &hd, const float *rgb
  * 513 KB 155 and 136, 2 MB 555 and 317, 32 MB 8.4 and 3.1 ms; one colour (66 values a byte, so the pixels
  * tell): 0.5 Mpixel 81 and 92, 2 Mpixel 160 and 120, 8 Mpixel 450 and 241.  Pieces of 64 to 256 KB are
  * slower and uneven (2 MB: 330 to 370 us), pinned ones 290, but pinning 1 MB costs a new context 1.3 ms. */
-constexpr size_t kHeadBytes = 1 << 16, kFilePiece = 1 << 20, kRowSmem = 200 << 10;
+constexpr size_t kFilePiece = 1 << 20, kRowSmem = 200 << 10;
 constexpr size_t kDeviceBytes = 5 << 16, kDevicePixels = 1 << 20;
 
 nova_b200_status read_rows_on_device(nova_b200_ctx *c, std::ifstream &f, const std::vector<unsigned char> &head,
-                                     size_t size, float *rgba_host, float *rgba_device, uint64_t capacity, bool *done) {
+                                     const Header &hd, size_t size, float *rgba_host, float *rgba_device,
+                                     uint64_t capacity, bool *done) {
   using namespace nbctx;
   *done = false;
-  if (size <= head.size()) return NOVA_B200_SUCCESS; /* the head is all of it */
-  Header hd;
-  if (parse_header(c, head, hd) || hd.data + 4 > head.size() || !rle_width(hd.w)) return NOVA_B200_SUCCESS;
+  if (size <= kHeadBytes || hd.data + 4 > head.size() || !rle_width(hd.w)) return NOVA_B200_SUCCESS;
   const uint32_t pattern = 2u | 2u << 8 | (uint32_t)(hd.w >> 8) << 16 | (uint32_t)(hd.w & 255) << 24;
   uint32_t word;
   std::memcpy(&word, &head[hd.data], 4);
@@ -762,9 +764,10 @@ nova_b200_status read_rows_on_device(nova_b200_ctx *c, std::ifstream &f, const s
   if (e == cudaSuccess) e = cudaMemsetAsync(d_body + n, 0, 256, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_ok, 0xff, sizeof(uint32_t) * (1 + (size_t)most), c->stream);
   bool read = true;
-  f.seekg((std::streamoff)hd.data);
-  const std::unique_ptr<char[]> piece(new char[(size_t)std::min<uint64_t>(n, kFilePiece)]);
-  for (uint64_t off = 0; e == cudaSuccess && read && off < n; off += kFilePiece) {
+  const uint64_t held = head.size() - hd.data; /* bytes of the body that have been read */
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_body, &head[hd.data], held, cudaMemcpyHostToDevice, c->stream);
+  const std::unique_ptr<char[]> piece(new char[(size_t)std::min<uint64_t>(n - held, kFilePiece)]);
+  for (uint64_t off = held; e == cudaSuccess && read && off < n; off += kFilePiece) {
     const size_t bytes = (size_t)std::min<uint64_t>(kFilePiece, n - off);
     read = (bool)f.read(piece.get(), (std::streamsize)bytes);
     if (read) e = cudaMemcpyAsync(d_body + off, piece.get(), bytes, cudaMemcpyHostToDevice, c->stream);
@@ -869,7 +872,7 @@ extern "C" nova_b200_status nova_b200_hdr_info(nova_b200_ctx *c, const char *pat
   std::vector<unsigned char> bytes;
   std::ifstream f;
   size_t size = 0;
-  nova_b200_status st = read_head(c, path, f, kHeadBytes, bytes, size);
+  nova_b200_status st = read_head(c, path, f, 0, bytes, size);
   if (st) return st;
   Header hd;
   st = parse_header(c, bytes, hd);
@@ -890,14 +893,22 @@ extern "C" nova_b200_status nova_b200_hdr_read(nova_b200_ctx *c, const char *pat
   std::ifstream f;
   std::vector<unsigned char> bytes;
   size_t size = 0;
-  nova_b200_status st = read_head(c, path, f, kHeadBytes, bytes, size);
+  /* a file that the host's walk takes unless it has many pixels is read at once: in two pieces, with the header
+   * parsed for each, 320 x 240 took 3 us more of 138 */
+  nova_b200_status st = read_head(c, path, f, kDeviceBytes, bytes, size);
   if (st) return st;
-  bool done = false;
-  st = read_rows_on_device(c, f, bytes, size, rgba_host, rgba_device, capacity, &done);
-  if (st || done) return st;
-  if ((st = read_rest(c, path, f, bytes, size))) return st;
   Header hd;
-  if ((st = parse_header(c, bytes, hd))) return st;
+  st = parse_header(c, bytes, hd);
+  if (!st) {
+    bool done = false;
+    st = read_rows_on_device(c, f, bytes, hd, size, rgba_host, rgba_device, capacity, &done);
+    if (st || done) return st;
+  }
+  if (bytes.size() < size) {
+    if ((st = read_rest(c, path, f, bytes, size))) return st;
+    st = parse_header(c, bytes, hd);
+  }
+  if (st) return st;
   if ((st = check_read(c, hd, rgba_device, capacity))) return st;
   const uint64_t npx = (uint64_t)hd.w * hd.h;
   Layout L;
