@@ -162,8 +162,8 @@ __device__ __forceinline__ V3 bake_sum(const Src &src, const float *lut, const T
   return irr;
 }
 
-/* G lanes per output texel.  Bound by instruction issue (84 % of the slots, 28 of 32 lanes): about 500 a
- * sample, 91 of them in double precision.  512 x 256 texels x 128 samples of a 2048 x 1024 map, one call:
+/* G lanes per output texel.  Bound by instruction issue (81 % of the slots, 28 of 32 lanes): about 380 a
+ * sample.  512 x 256 texels x 128 samples of a 2048 x 1024 map, one call:
  * 507 us with four texel loads and five double-precision functions a sample, 264 us with one load and
  * three (the source read for non-finite texels included).  256 x 128 texels, where one thread per texel
  * fills a tenth of the GPU: 347 us with one lane, 99 with eight. */

@@ -681,9 +681,9 @@ __global__ void __launch_bounds__(kBlock) k_partition(Shared s, int level) {
  * lanes compute them or in which order, so the tree is the one a single warp building node after
  * node produces.
  *
- * Bound by chains of dependent shuffles and shared-memory loads at 28 warps per SM.  163 k triangles:
- * sorting every node and loading its boxes from memory again took 195 us, this 133 (62 M warp
- * instructions, 53 % of the issue slots). */
+ * Bound by chains of dependent shuffles and shared-memory loads at 23 warps per SM (58 % of the issue slots, 64 M
+ * warp instructions).  163 k triangles: sorting every node and loading its boxes from memory again took 195 us,
+ * this 133. */
 /* Right siblings a W-lane segment keeps: it pushes only at nodes of >= W / 2 + 2 primitives (smaller
  * ones fork), nested with strictly decreasing sizes <= W, so at most W / 2 - 1 at once (none for
  * W <= 2).  Per warp: one segment of 32 lanes (15 entries), 2 of 16 (7 each), 4 of 8 (3 each) and 8

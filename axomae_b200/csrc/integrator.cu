@@ -16,6 +16,9 @@
  *   k_resolve  per pixel, adds the per-path radiance of the call's samples to the running sum in
  *              sample order and writes sum / samples (writeFramebuffer, api/engine.cpp:351-363)
  *
+ * The steps of a path are in wavefront.cuh; the adjoint's waves (wave_adjoint.cu) and trace modes 1 to 3
+ * (wave_modes.cu) are modules of their own.
+ *
  * Jobs: every path carries its job index (a frame of one context: scene, BVH, camera, sample
  * range) and every kernel reads the chunk's job table, so a batch of frames of different scenes
  * runs as one wavefront.  A single render is a batch of one.  The table travels in the kernel

@@ -140,7 +140,7 @@ NB_D bool visit_tri(const Rec &q, V3 o, V3 d, float tmax, float &t, float &u, fl
 
 /* Closest hit of one world-space ray on the binary BVH.
  *
- * Bound by instruction issue at 17 of 32 active lanes and by the latency of dependent loads (issue
+ * Bound by instruction issue at 16 of 32 active lanes and by the latency of dependent loads (issue
  * slots 67 % used on full waves; L1 60 %, DRAM 12 %).  One iteration visits a node or one triangle of a
  * leaf, and both kinds of lane load their record before the branch: a warp with lanes of each kind
  * waits for one load instead of two.  The slab distances are packed pairs (12 instructions a node

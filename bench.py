@@ -57,12 +57,12 @@ BATCH_METRIC = ("Mrays/s batched wavefront (32-job batch; plain wavefront on the
 
 
 # DRAM bytes per traced ray that ncu measured for k_trace (dram__bytes_read.sum +
-# dram__bytes_write.sum over full waves of 8,388,608 rays): batched workload waves 1-2, and the
-# heightfield's first wave (camera rays only).
-K_TRACE_DRAM_BYTES_PER_RAY = {"batched": 72.0, "heightfield": 238.4, "instanced": None}
+# dram__bytes_write.sum over full waves of 8,388,608 rays): batched workload waves 5-7, and the
+# heightfield's first wave (camera rays only).  Both include the camera rays the pass makes and queues.
+K_TRACE_DRAM_BYTES_PER_RAY = {"batched": 90.0, "heightfield": 129.5, "instanced": None}
 # L2 bytes per traced ray (lts__t_bytes.sum) ncu measured for the binary-BVH k_trace on the
-# batched workload's full waves 6-8: L1 serves ~2/3 of the requests, L2 ~90 % of the rest.
-K_TRACE_L2_BYTES_PER_RAY = {"batched": 521.0, "heightfield": None, "instanced": None}
+# batched workload's full waves 5-7.
+K_TRACE_L2_BYTES_PER_RAY = {"batched": 589.0, "heightfield": None, "instanced": None}
 
 
 def peaks():
@@ -476,8 +476,8 @@ def film_io_timing(local_rank, cpu_baseline=True, reps=10):
                                         "packing, D2H of the packed bytes, file write"}
         out["hdr_read_e2e"] = {"seconds": float(np.median(reads)), "mpix_per_s": W * H / float(np.median(reads)) / 1e6,
                                "h2d_bytes": int(file_mb * 1e6), "d2h_bytes": px_bytes,
-                               "note": "nova_b200_hdr_read to host pixels, wall clock: file read, packet-header scan "
-                                       "on the host, H2D of the file, device expansion and decode, D2H"}
+                               "note": "nova_b200_hdr_read to host pixels, wall clock: file read, H2D of the file, "
+                                       "rows found, expanded and decoded on the device, D2H"}
         if cpu_baseline:
             ob = oracle_module()
             t0 = time.perf_counter()
