@@ -204,8 +204,8 @@ nova_b200_status nova_b200_upload_build_batch(nova_b200_ctx *const *ctxs, const 
                                               uint32_t n, const nova_b200_bvh_options *opts);
 
 /* Renders one frame batch (renderGpu, api/engine.cpp:457-496).  film_host (width*height*4 floats,
- * pageable or pinned) and/or film_device (a device pointer) receive the running-mean RGBA image;
- * either may be NULL.  stats may be NULL. */
+ * pageable or pinned) and/or film_device (a device pointer; memory of another GPU is reached by a copy)
+ * receive the running-mean RGBA image; either may be NULL.  stats may be NULL. */
 nova_b200_status nova_b200_render(nova_b200_ctx *ctx, const nova_b200_frame *frame, float *film_host,
                                   float *film_device, nova_b200_render_stats *stats);
 
@@ -214,7 +214,8 @@ nova_b200_status nova_b200_render(nova_b200_ctx *ctx, const nova_b200_frame *fra
  * count and depth (no counterpart in the reference, which renders one engine at a time).  Every
  * frame follows the semantics of nova_b200_render on its own context (sample range, running-mean
  * film, reset) and produces the same film bit for bit.  films_host / films_device may be NULL or
- * hold n pointers (entries may be NULL).  All contexts must share a device and a BVH width.  When
+ * hold n pointers (entries may be NULL; device films may share memory, host films get their own frame's
+ * all the same).  All contexts must share a device and a BVH width.  When
  * the batch takes several chunks (more than 104 frames, or more paths than one radiance buffer
  * holds), the films of frames finished in an earlier chunk are copied out on a second stream while
  * later chunks render, if they are device or pinned host buffers; pageable ones are written at the
